@@ -13,7 +13,7 @@
 #pragma once
 
 template <int MODE, bool MIX>
-__global__ void __launch_bounds__(NTHREADS, SMAUG_MINB2D)
+__global__ void __launch_bounds__(NTHREADS, MIX ? SMAUG_MINB2D_MIX : SMAUG_MINB2D)
     stage2d_batch(const KParams* __restrict__ Ks, const KBufs* __restrict__ Bs,
                   const int4* __restrict__ tiles, int ntiles) {
   for (int it = blockIdx.x; it < ntiles; it += gridDim.x) {
@@ -65,7 +65,7 @@ __device__ __forceinline__ bool batch_grid_sync(BatchSync* s, int* err, unsigned
 // on the GPU at once.  Stage inputs written by other blocks earlier in the
 // launch are read through L2 (the CG form of the stage body).
 template <bool MIX>
-__global__ void __launch_bounds__(NTHREADS, SMAUG_MINB2D)
+__global__ void __launch_bounds__(NTHREADS, MIX ? SMAUG_MINB2D_MIX : SMAUG_MINB2D)
     stage2d_batch_cycle(const KParams* __restrict__ Ks, const KBufs* __restrict__ Bs,
                         const int4* __restrict__ tiles, int ntiles, int nruns, int k0, int nsteps,
                         BatchSync* sync, int* err) {

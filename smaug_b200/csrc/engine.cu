@@ -461,7 +461,7 @@ static int create(const smaug_params_t* p, const double* w, const double* pos, E
       if (e->d_u[i]) ok = stage2d_tma_encode(&e->tm_u[i], e->d_u[i], false, e->K, e->nevo, e->nevo) == 0;
     for (int i = 0; i < 4 && ok; i++)
       if (e->d_h[i]) ok = stage2d_tma_encode(&e->tm_h[i], e->d_h[i], true, e->K, e->nevo, e->nevo) == 0;
-    if (ok) ok = stage2d_tma_encode(&e->tm_bg, e->d_bg, false, e->K, e->nbg, e->K.has_bg ? 4 : 1) == 0;
+    if (ok) ok = stage2d_tma_encode(&e->tm_bg, e->d_bg, false, e->K, e->nbg, 1) == 0;
     e->tma_ok = ok;
     e->tma = 0;
   }

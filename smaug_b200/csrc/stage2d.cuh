@@ -1,12 +1,18 @@
-// stage2d.cuh -- fused 2D stage kernel, included by stage2d.cu.
+// stage2d.cuh -- fused 2D stage kernel, included by stage2d.cu,
+// stage2d_tma.cu, batch.cu and batch16.cu (each with its tile constants).
 //
-// One launch evaluates the reference's whole spatial operator for a 32x8
+// One launch evaluates the reference's whole spatial operator for a TX x TY
 // tile of interior cells and writes the stage result, its ghost images and
-// the per-dimension fast-speed maxima.  Term by term it follows the launch
-// order of the reference's step (src/iosmaug.c:631-835); the arithmetic of
-// each term is the reference's, with divisions by rho_t and by the cell
-// width replaced by multiplications with per-cell / per-line reciprocals
-// (agreement with the reference stays at rounding level, ~1e-16 relative).
+// the per-dimension fast-speed maxima.  The terms are those of the
+// reference's step (src/iosmaug.c:631-835); sums are regrouped at rounding
+// level (agreement with the reference stays ~1e-16 relative):
+//   - divisions by rho_t and by the cell width are multiplications with
+//     reciprocals;
+//   - the source of a hyperdiffusion pass is a difference of face fluxes: with
+//     R(i) = max|D3| / max|D1| the reference's coefficients are nu_r(i) = c(i)
+//     R(i), nu_l(i) = c(i) R(i-1), c = dl cmax chyp, so that the pass adds dt
+//     cmax/dl (G(i) - G(i-1)) with G(i) = chyp R(i) (q(i+1) - q(i)) x face mean;
+//   - increments are summed from zero and added to the base state.
 //
 // Two precision forms share the code (template MIX):
 //   FP64   every value and every operation in double;
@@ -14,413 +20,350 @@
 //          state as a float high/low pair), backgrounds in double; fluxes,
 //          the pressure recovery p_t = (g-1)(e - m^2/2rho_t) - ..., the
 //          CFL speeds, the stage sums and the RK4 accumulator in double;
-//          the hyperdiffusion coefficient and sources (q, nu, their
-//          differences) in float, with q itself formed in double.
+//          the hyperdiffusion ratios and face fluxes in float, with q itself
+//          formed in double and every pass's increment summed in double.
 //
-// Shared memory: the tile's state (6 perturbation fields in the storage
-// type, the background fields in double) on the tile + 3-cell halo, 1/rho_t,
-// the tile's cell widths and their reciprocals, then one union of phase
-// scratch:
-//   flux phase:  5 flux arrays on the tile +-2 cells along the direction
-//                (+ 2 velocity arrays when background fields are present)
-//   hyperdiffusion phase: q of one field on the whole region (shared by the
-//                passes of both directions), the nu ratio on the tile
-//                extended by one cell along the direction, two cross-term
-//                arrays on the tile +-1 across.
+// A block works in phases over the tile, all fields and both directions per
+// phase, so that it meets five block barriers:
+//   0  staging: q of the six hyperdiffusion fields on the tile + 3-cell halo
+//   1  centred fluxes of both directions on the tile +-2
+//   2  own cell: divergence of the fluxes, background coupling, gravity
+//   3  nu ratios of all ten passes; one thread takes a line of a field (11
+//      faces along x, the tile's height along y) through running windows
+//      (RatioWindow): 14 to 16 loads per line instead of six per face
+//   4  cross-term arrays of the four passes that have them
+//   5  own cell: diffusive and cross terms, driver, stage sum, stores, ghost
+//      images, CFL maxima
+// The arrays of phases 1-2 and 3-5 share their memory.
 #pragma once
 
 // (included inside namespace smaug)
 namespace s2 {
-// flux arrays: the tile +-2 along the direction (+-3 along dim 0 for the
-// 6th-order derivative, which a 2D build of the reference applies along dim 0
-// only: its dir-1 USE_DORDER3 branch is overwritten by the 4th-order form,
-// src/gradops.cu:536-544)
-template <bool O6>
-__host__ __device__ constexpr int fsz() {
-  return (TX + (O6 ? 6 : 4)) * TY > TX * (TY + 4) ? (TX + (O6 ? 6 : 4)) * TY : TX * (TY + 4);
-}
-constexpr int RSZ = (TX + 1) * (TY + 2) > (TX + 2) * (TY + 1) ? (TX + 1) * (TY + 2) : (TX + 2) * (TY + 1);
-constexpr int NSZ = TX * (TY + 2) > (TX + 2) * TY ? TX * (TY + 2) : (TX + 2) * TY;
-constexpr int HYP = RC + RSZ + 2 * NSZ;  // q, ratio, two cross-term arrays
-template <bool MIX, bool O6 = false>
-__host__ __device__ constexpr size_t union_bytes() {
-  return (5 * fsz<O6>() * sizeof(double)) > HYP * sizeof(typename Form<MIX>::H)
-             ? 5 * fsz<O6>() * sizeof(double)
-             : HYP * sizeof(typename Form<MIX>::H);
-}
+// rows of the staged arrays: an odd pitch, so that lines along x taken by
+// neighbouring threads fall on different banks
+constexpr int QX = RX | 1;
+constexpr int QC = QX * RY;
+// staged fields: q of rho, e, v1, v2, b1, b2; the mixed form also keeps the
+// momenta and the energy as stored (floats), which products with 1/rho_t would
+// round again
+enum { QR = 0, QE = 1, QV1 = 2, QV2 = 3, QB1 = 4, QB2 = 5, QM1 = 6, QM2 = 7, QEN = 8 };
+template <bool BG, bool MIX, bool O6>
+struct Lay {
+  using H = typename Form<MIX>::H;
+  static constexpr int NQ = MIX ? 9 : 6;
+  static constexpr int NC = MIX ? 4 : 3;     // cross arrays: m, B, energy (v and b parts)
+  // flux arrays: the tile +-2 along the direction (+-3 along dim 0 for the
+  // 6th-order derivative, which a 2D build of the reference applies along
+  // dim 0 only: its dir-1 USE_DORDER3 branch is overwritten by the 4th-order
+  // form, src/gradops.cu:536-544)
+  static constexpr int FH = O6 ? 3 : 2;
+  static constexpr int FXW = TX + 2 * FH, FXN = FXW * TY, FYN = TX * (TY + 4);
+  // ratio arrays of the five passes along x (faces -1 .. TX-1, rows -1 .. TY)
+  // and along y (columns -1 .. TX, faces -1 .. TY-1); cross arrays on the tile
+  // +-1 across
+  static constexpr int RXW = TX + 1, RXN = RXW * (TY + 2), RYW = TX + 2, RYN = RYW * (TY + 1);
+  static constexpr int CXN = TX * (TY + 2), CYW = TX + 2, CYN = CYW * TY;
+  // byte offsets; double arrays first
+  static constexpr int RT = 0;                                  // rho_t (background fields only)
+  static constexpr int RI = RT + (BG ? QC * 8 : 0);             // 1/rho_t (mixed only)
+  static constexpr int RD = RI + (MIX ? QC * 8 : 0);            // 1/dl of the region's columns and rows
+  static constexpr int U = RD + (RX + RY) * 8;                  // union
+  static constexpr int FB = 5 * (FXN + FYN) * 8;
+  static constexpr int HB = (5 * (RXN + RYN) + NC * (CXN + CYN)) * (int)sizeof(H);
+  static constexpr int Q = U + ((FB > HB ? FB : HB) + 15) / 16 * 16;
+  static constexpr int BYTES = Q + NQ * QC * (int)sizeof(H);
+};
 template <bool BG, bool MIX, bool O6 = false>
 __host__ __device__ constexpr size_t smem_bytes() {
-  return 6 * RC * sizeof(typename Form<MIX>::S) +
-         sizeof(double) * ((BG ? 6 : 0) * RC + RC + 2 * (RX + RY)) + union_bytes<MIX, O6>();
+  return Lay<BG, MIX, O6>::BYTES;
 }
-}  // namespace s2
 
-template <bool BG, bool MIX>
-struct T2 {
-  using ST = typename Form<MIX>::S;
-  ST* S;         // [6][RC] perturbation state
-  double* G;     // [4][RC] background fields (BG only)
-  double* R;     // [RC] 1/rho_t
-  double* V;     // [2][RC] velocities (BG only)
-  double* dl0;   // [RX] widths along x of the region columns
-  double* dl1;   // [RY]
-  double* rd0;   // [RX] reciprocals
-  double* rd1;   // [RY]
-  void* U;       // union scratch
-  int x0, y0;
-  bool inner;    // the staged region lies inside the grid and off its pads
-  // field f of the reference numbering at region cell l, in double
-  __device__ __forceinline__ double v(int f, int l) const {
-    if (f < 6) return (double)S[f * RC + l];
-    return BG ? G[(f - 6) * RC + l] : 0.0;
+// derived values of one region cell (r: its index in the staged arrays)
+template <bool BG, bool MIX, bool O6, typename ST>
+__device__ __forceinline__ void derive(char* sm, int r, bool ok, const ST* w, double rhob) {
+  using L = Lay<BG, MIX, O6>;
+  using HT = typename L::H;
+  HT* const Q = reinterpret_cast<HT*>(sm + L::Q);
+  const double m1 = (double)w[M1], m2 = (double)w[M2], b1 = (double)w[B1], b2 = (double)w[B2];
+  double rt = BG ? (double)w[RHO] + rhob : (double)w[RHO];
+  if (!ok) rt = 1.0;
+  const double ri = recip(rt);
+  const double v1 = m1 * ri, v2 = m2 * ri;
+  Q[QR * QC + r] = (HT)w[RHO];
+  Q[QE * QC + r] = (HT)((double)w[EN] - 0.5 * ((b1 * b1 + b2 * b2) + (m1 * v1 + m2 * v2)));
+  Q[QV1 * QC + r] = (HT)v1;
+  Q[QV2 * QC + r] = (HT)v2;
+  Q[QB1 * QC + r] = (HT)w[B1];
+  Q[QB2 * QC + r] = (HT)w[B2];
+  if constexpr (MIX) {
+    Q[QM1 * QC + r] = (HT)w[M1];
+    Q[QM2 * QC + r] = (HT)w[M2];
+    Q[QEN * QC + r] = (HT)w[EN];
+    reinterpret_cast<double*>(sm + L::RI)[r] = ri;
   }
-};
+  if (BG) reinterpret_cast<double*>(sm + L::RT)[r] = rt;
+}
 
 // fluxes along D of rho, m1, m2, e and the B component across D at region
-// cell l (src/centdiff1.cu:51-197, src/centdiff2.cu:203-323):
+// cell r (src/centdiff1.cu:51-197, src/centdiff2.cu:203-323):
 //   F_rho = m_D (= m_D rho'/rho_t + rho_b m_D/rho_t)
 //   F_m_c = v_D m_c + delta_cD p_t - (B'_c Bb_D + Bb_c B'_D) - B'_c B'_D
 //   F_e   = v_D (e + p_t + e_b) - (B'_D (Bb.m) + Bb_D (B'.m) + B'_D (B'.m)) / rho_t
 //   F_B_c = v_D (B'_c + Bb_c) - v_c (B'_D + Bb_D)
-template <bool BG, bool MIX, int D>
-__device__ __forceinline__ void flux_at(const T2<BG, MIX>& T, double gamma, int l, double* F) {
-  const double m1 = T.v(M1, l), m2 = T.v(M2, l);
-  const double e = T.v(EN, l), b1 = T.v(B1, l), b2 = T.v(B2, l);
-  double eb = 0, bb1 = 0, bb2 = 0;
-  if (BG) {
-    eb = T.v(EB, l);
-    bb1 = T.v(BB1, l);
-    bb2 = T.v(BB2, l);
+// In the FP64 form e and p_t come from the staged q_e = e - (B'^2 + m.v)/2:
+// p_t = (g-1)(q_e + B'^2/2) - (g-2)(B'.Bb + B'^2/2).
+template <bool BG, bool MIX, bool O6, int D>
+__device__ __forceinline__ void flux_at(const char* sm, double gamma, int r, const double* g, double* F) {
+  using L = Lay<BG, MIX, O6>;
+  using HT = typename L::H;
+  const HT* const Q = reinterpret_cast<const HT*>(sm + L::Q);
+  const double b1 = (double)Q[QB1 * QC + r], b2 = (double)Q[QB2 * QC + r];
+  double m1, m2, v1, v2, e, msr;
+  const double hb = 0.5 * (b1 * b1 + b2 * b2);
+  if constexpr (MIX) {
+    const double ri = reinterpret_cast<const double*>(sm + L::RI)[r];
+    m1 = (double)Q[QM1 * QC + r];
+    m2 = (double)Q[QM2 * QC + r];
+    v1 = m1 * ri;
+    v2 = m2 * ri;
+    msr = 0.5 * (m1 * v1 + m2 * v2);
+    e = (double)Q[QEN * QC + r] - msr;
+  } else {
+    const double rt = BG ? reinterpret_cast<const double*>(sm + L::RT)[r] : (double)Q[QR * QC + r];
+    v1 = (double)Q[QV1 * QC + r];
+    v2 = (double)Q[QV2 * QC + r];
+    m1 = v1 * rt;
+    m2 = v2 * rt;
+    msr = 0.5 * (m1 * v1 + m2 * v2);
+    e = (double)Q[QE * QC + r] + hb;
   }
-  const double r = T.R[l];
-  const double md = D == 0 ? m1 : m2;
-  const double vd = md * r;
-  // computept3 (src/dervfields.cu:107-153)
-  const double pt = (gamma - 1.0) * (e - 0.5 * (m1 * m1 + m2 * m2) * r) -
-                    (gamma - 2.0) * ((b1 * bb1 + b2 * bb2) + 0.5 * (b1 * b1 + b2 * b2));
-  const double bd = D == 0 ? b1 : b2, bbd = D == 0 ? bb1 : bb2;
+  const double bb1 = BG ? g[2] : 0.0, bb2 = BG ? g[3] : 0.0;
+  // computept3 (src/dervfields.cu:107-153); e holds the energy without m.v/2
+  const double pt = (gamma - 1.0) * e - (gamma - 2.0) * (BG ? (b1 * bb1 + b2 * bb2) + hb : hb);
+  const double md = D == 0 ? m1 : m2, vd = D == 0 ? v1 : v2, bd = D == 0 ? b1 : b2;
+  const double bbd = D == 0 ? bb1 : bb2;
+  const double t1 = BG ? b1 + bb1 : b1, t2 = BG ? b2 + bb2 : b2, td = D == 0 ? t1 : t2;
+  const double bv = b1 * v1 + b2 * v2;
+  const double tv = BG ? bv + (bb1 * v1 + bb2 * v2) : bv;  // (B' + B_b) . v
   F[0] = md;
-  // momentum components
-  F[1] = vd * m1 + (D == 0 ? pt : 0.0) - (b1 * bbd + bb1 * bd) - b1 * bd;
-  F[2] = vd * m2 + (D == 1 ? pt : 0.0) - (b2 * bbd + bb2 * bd) - b2 * bd;
-  // energy
-  const double bbm = bb1 * m1 + bb2 * m2, bm = b1 * m1 + b2 * m2;
-  F[3] = vd * (e + pt + eb) - (bd * bbm + bbd * bm + bd * bm) * r;
-  // B component across D
-  if (D == 0)
-    F[4] = vd * (b2 + bb2) - (m2 * r) * (b1 + bb1);
-  else
-    F[4] = vd * (b1 + bb1) - (m1 * r) * (b2 + bb2);
+  F[1] = vd * m1 + (D == 0 ? pt : 0.0) - (BG ? b1 * td + bb1 * bd : b1 * bd);
+  F[2] = vd * m2 + (D == 1 ? pt : 0.0) - (BG ? b2 * td + bb2 * bd : b2 * bd);
+  F[3] = vd * ((e + msr) + pt + (BG ? g[0] : 0.0)) - (BG ? bd * tv + bbd * bv : bd * bv);
+  F[4] = D == 0 ? v1 * t2 - v2 * t1 : v2 * t1 - v1 * t2;
 }
 
-// q of a hyperdiffusion pass at region cell l (src/hyperdifvisc1r.cu:1225-1253),
-// formed in double
-template <bool BG, bool MIX, int KIND, int COMP>
-__device__ __forceinline__ double hq_at(const T2<BG, MIX>& T, int l) {
-  if (KIND == 0) return T.v(RHO, l);
-  if (KIND == 1) {
-    const double m1 = T.v(M1, l), m2 = T.v(M2, l);
-    const double b1 = T.v(B1, l), b2 = T.v(B2, l);
-    return T.v(EN, l) - 0.5 * ((b1 * b1 + b2 * b2) + (m1 * m1 + m2 * m2) * T.R[l]);
-  }
-  if (KIND == 2) return T.v(M1 + COMP, l) * T.R[l];
-  return T.v(B1 + COMP, l);
-}
-
-// the same q from global memory (stray pad source cell)
-template <typename ST, int KIND, int COMP, bool CG = false>
-__device__ __forceinline__ double hq_global(const ST* u, const double* bg, long nc, long c) {
-  auto ld = [&](long i) { return CG ? (double)__ldcg(u + i) : (double)u[i]; };
-  const double rho = ld(0 * nc + c), rhob = bg[1 * nc + c];
-  if (KIND == 0) return rho;
-  const double r = 1.0 / (rho + rhob);
-  if (KIND == 1) {
-    const double m1 = ld(1 * nc + c), m2 = ld(2 * nc + c);
-    const double b1 = ld(4 * nc + c), b2 = ld(5 * nc + c);
-    return ld(3 * nc + c) - 0.5 * ((b1 * b1 + b2 * b2) + (m1 * m1 + m2 * m2) * r);
-  }
-  if (KIND == 2) return ld((1 + COMP) * nc + c) * r;
-  return ld((4 + COMP) * nc + c);
-}
-
-// (A) q of one hyperdiffusion field on the whole staged region, with the
-// reference's pads: index -1 along an axis holds the copy of index 5
-// (bc_hyperdifl), index n the stray tmp6 store of hyperdifvisc1r_parallel
-// (source table B.padsrc).  The passes of both directions read it.
-template <bool BG, bool MIX, int KIND, int COMP, bool CG = false>
-__device__ __forceinline__ void stage_q2(const T2<BG, MIX>& T, const KParams& P, const KBufs& B,
-                                         int tid) {
-  using HT = typename Form<MIX>::H;
-  using ST = typename Form<MIX>::S;
-  HT* Q = static_cast<HT*>(T.U);
-  const int n0 = P.n0, n1 = P.n1;
-  const long nc = P.ncell;
-  if (T.inner) {
-    for (int u = tid; u < RXU * RY; u += NTHREADS) {
-      const int r = RXU == RX ? u : (u / RXU) * RX + u % RXU;
-      Q[r] = (HT)hq_at<BG, MIX, KIND, COMP>(T, r);
-    }
-    __syncthreads();
-    return;
-  }
-  for (int u = tid; u < RXU * RY; u += NTHREADS) {
-    const int lx = u % RXU, ly = u / RXU, r = ly * RX + lx;
-    const int ci = T.x0 - HALO + lx, cj = T.y0 - HALO + ly;
-    const bool inx = ci >= 0 && ci < n0, iny = cj >= 0 && cj < n1;
-    double q = 0.0;
-    if (inx && iny) {
-      q = hq_at<BG, MIX, KIND, COMP>(T, r);
-    } else if (iny) {
-      if (ci == -1) {
-        q = hq_at<BG, MIX, KIND, COMP>(T, r + 6);
-      } else if (ci == n0) {
-        const int src = B.padsrc[0][cj];
-        if (src >= 0) q = hq_global<ST, KIND, COMP, CG>(static_cast<const ST*>(B.uin), B.bg, nc, src);
-      }
-    } else if (inx) {
-      if (cj == -1) {
-        q = hq_at<BG, MIX, KIND, COMP>(T, r + 6 * RX);
-      } else if (cj == n1) {
-        const int src = B.padsrc[1][ci];
-        if (src >= 0) q = hq_global<ST, KIND, COMP, CG>(static_cast<const ST*>(B.uin), B.bg, nc, src);
-      }
-    }
-    Q[r] = (HT)q;
-  }
-  __syncthreads();
-}
-
-// One hyperdiffusion pass on staged q: field kind (0 rho, 1 energy,
-// 2 momentum, 3 B), component COMP, direction DIM.
-//
-// nu_r and nu_l (hyperdifvisc2-4) are ratios of windowed maxima of the third
-// differences D3 and first differences D1 of q:
-//   nu_r(i) = dl(i) cmax chyp max D3(i-1..i+1) / max D1(i-2..i+2)
-//   nu_l(i) = dl(i) cmax chyp max D3(i-2..i)   / max D1(i-3..i+1)
-// (0 where the denominator is 0, and 0 outside [2, n-3] in every
-// dimension).  The windows of nu_l(i) are those of nu_r(i-1), so one ratio
-// R(i) = max D3 / max D1 per cell serves both: nu_r(i) = c(i) R(i),
-// nu_l(i) = c(i) R(i-1).
-template <bool BG, bool MIX, int KIND, int COMP, int DIM>
-__device__ __forceinline__ void hyper_pass(const T2<BG, MIX>& T, const KParams& P, const KBufs& B,
-                                           int tid, bool active, int lxo, int lyo, int gi, int gj,
-                                           double dt, const double* cin, double* out) {
-  using HT = typename Form<MIX>::H;
-  constexpr int SX = (DIM == 0), SY = (DIM == 1);
-  constexpr int QFIELD = (KIND == 0) ? RHO : (KIND == 1) ? EN : (KIND == 2) ? M1 + COMP : B1 + COMP;
-  constexpr bool CROSS = (KIND == 2 && COMP != DIM) || (KIND == 3);
-  const int n0 = P.n0, n1 = P.n1;
-  const int nd = DIM == 0 ? n0 : n1;
-  const HT* Q = static_cast<const HT*>(T.U);  // region-indexed q
-  HT* RR = static_cast<HT*>(T.U) + RC;         // ratio area
-  HT* C3 = RR + s2::RSZ;                       // cross-term arrays (nu area)
-  HT* C4 = C3 + s2::NSZ;
-  constexpr int SQ = DIM == 0 ? 1 : RX;        // stride along DIM in Q
-  // ratio area: the tile along DIM extended by one cell below, the tile
-  // across (+-1 when cross terms need it)
-  constexpr int exR = DIM == 0 ? TX + 1 : (CROSS ? TX + 2 : TX);
-  constexpr int eyR = DIM == 0 ? (CROSS ? TY + 2 : TY) : TY + 1;
-  constexpr int oxR = DIM == 0 ? HALO - 1 : (CROSS ? HALO - 1 : HALO);
-  constexpr int oyR = DIM == 0 ? (CROSS ? HALO - 1 : HALO) : HALO - 1;
-  constexpr int SR = DIM == 0 ? 1 : exR;       // stride along DIM in RR
-  // nu area: the tile along DIM, +-1 across
-  constexpr int exN = (DIM == 0) ? TX : TX + 2, eyN = (DIM == 0) ? TY + 2 : TY;
-  constexpr int oxN = (DIM == 0) ? HALO : HALO - 1, oyN = (DIM == 0) ? HALO - 1 : HALO;
-  auto ri = [&](int lx, int ly) { return (ly - oyR) * exR + (lx - oxR); };
-  auto ni = [&](int lx, int ly) { return (ly - oyN) * exN + (lx - oxN); };
-  const HT coef = (HT)(cin[DIM] * P.chyp[QFIELD]);
-
-  // (B) R = max D3(i-1..i+1) / max D1(i-2..i+2) from q(i-2..i+3)
-  for (int r = tid; r < exR * eyR; r += NTHREADS) {
-    const int lx = oxR + r % exR, ly = oyR + r / exR;
-    const int l = ly * RX + lx;
-    HT q[6];
+// N faces of a line of q, stride S: the ratios of faces l0 .. l0+N-1 from q(l0-2
+// .. l0+N+2); put(k, R, q(l+1) - q(l)) takes face l0 + k.  Faces from n on are
+// left out (the last piece of a row may be shorter).
+template <int N, int S, bool FULL, typename H, typename Put>
+__device__ __forceinline__ void ratio_line(const H* q, int n, Put put) {
+  RatioWindow<H> w{};
+  H a1 = 0, a2 = 0, a3 = 0;  // q one, two and three cells back
 #pragma unroll
-    for (int s = 0; s < 6; s++) q[s] = Q[l + (s - 2) * SQ];
-    HT t4 = 0, t5 = 0;
-#pragma unroll
-    for (int k = 0; k < 3; k++)
-      t4 = hmax0(t4, (HT)fabs((HT)3 * (q[k + 2] - q[k + 1]) - (q[k + 3] - q[k])));
-#pragma unroll
-    for (int k = 0; k < 5; k++) t5 = hmax0(t5, (HT)fabs(q[k + 1] - q[k]));
-    RR[r] = (t5 > 0) ? hdiv(t4, t5) : (HT)0;
-  }
-  __syncthreads();
-  // (C) cross-term arrays (hyperdifmomsourcene2-4 / hyperdifbsourcene1b-4)
-  if (CROSS) {
-    for (int r = tid; r < exN * eyN; r += NTHREADS) {
-      const int lx = oxN + r % exN, ly = oyN + r / exN;
-      const int ci = T.x0 - HALO + lx, cj = T.y0 - HALO + ly;
-      HT c3 = 0, c4 = 0;
-      if (T.inner || (ci > 0 && ci < n0 - 1 && cj > 0 && cj < n1 - 1)) {
-        const int a = DIM == 0 ? ci : cj;
-        const int l = ly * RX + lx;
-        // grad13n along DIM of q
-        HT g = ((Q[l + SQ] - Q[l - SQ]) * (HT)(DIM == 0 ? T.rd0[lx] : T.rd1[ly])) * (HT)0.5;
-        if ((P.bt[DIM] != 0) && zero1n(a, nd)) g = 0;
-        HT nsum = 0;
-        if (T.inner || (ci >= 2 && ci <= n0 - 3 && cj >= 2 && cj <= n1 - 3)) {
-          const int rr = ri(lx, ly);
-          const HT c = (HT)(DIM == 0 ? T.dl0[lx] : T.dl1[ly]) * coef;
-          nsum = c * RR[rr] + c * RR[rr - SR];
-        }
-        if (KIND == 2) {
-          const HT tau = (g * nsum) * (HT)0.25;
-          c3 = (HT)(T.v(RHO, l) + T.v(RHOB, l)) * tau;
-          c4 = tau * (HT)T.v(M1 + DIM, l);
-        } else {
-          const HT t3 = (g * nsum) * (HT)0.5;
-          c3 = t3;
-          c4 = t3 * (HT)T.v(B1 + DIM, l);
-        }
-      }
-      C3[r] = c3;
-      C4[r] = c4;
+  for (int k = 0; k < N + 5; k++) {
+    if (FULL || k < n + 5) {
+      const H a = q[(k - 2) * S];
+      H t5 = 0, t4 = 0;
+      if (k >= 1) w.d1(a, a1, t5);
+      if (k >= 3) w.d3(a, a1, a2, a3, t4);
+      if (k >= 5) put(k - 5, nu_ratio(t4, t5), a2 - a3);
+      a3 = a2;
+      a2 = a1;
+      a1 = a;
     }
-    __syncthreads();
   }
-  // (D) sources at the tile cells (all inside [2, n-3])
-  if (active) {
-    const int a = DIM == 0 ? gi : gj;
-    const int l = lyo * RX + lxo;
-    const int rr = ri(lxo, lyo);
-    const int nidx = ni(lxo, lyo);
-    const HT c = (HT)(DIM == 0 ? T.dl0[lxo] : T.dl1[lyo]) * coef;
-    const HT nur = c * RR[rr], nul = c * RR[rr - SR];
-    const HT rdl = (HT)(DIM == 0 ? T.rd0[lxo] : T.rd1[lyo]);
-    const HT qc = Q[l], qp = Q[l + SQ], qm = Q[l - SQ];
-    HT gr = (qp - qc) * rdl;   // grad1r3n
-    HT gl = (qc - qm) * rdl;   // grad1l3n
-    if ((P.bt[DIM] != 0) && zero1n(a, nd)) { gr = 0; gl = 0; }
-    constexpr int SL = SX + SY * RX;  // region stride along DIM
-    if (KIND == 0) {
-      out[RHO] = out[RHO] + dt * (double)((nur * gr - nul * gl) * rdl);
-    } else if (KIND == 1) {
-      out[EN] = out[EN] + dt * (double)((nur * gr - nul * gl) * rdl);
-    } else if (KIND == 2) {
-      // hyperdifmomsource1-3a (src/hyperdifmomsource1.cu:17-511), ii0 = COMP
-      const double rb0 = T.v(RHOB, l), rbm = T.v(RHOB, l - SL), rbp = T.v(RHOB, l + SL);
-      const double r0 = T.v(RHO, l);
-      const HT t2 = (HT)((r0 + rb0 + T.v(RHO, l - SL) + rbm) * 0.5);
-      const HT t3 = (HT)((r0 + rb0 + T.v(RHO, l + SL) + rbp) * 0.5);
-      const double mf = T.v(M1 + COMP, l);
-      const HT t5 = (HT)((mf + T.v(M1 + COMP, l - SL)) * 0.5);
-      const HT t6 = (HT)((mf + T.v(M1 + COMP, l + SL)) * 0.5);
-      const double dm = (double)(((t3 * nur * gr - t2 * nul * gl) * rdl) * (HT)0.5);
-      const double de = (double)(((t6 * nur * gr - t5 * nul * gl) * rdl) * (HT)0.5);
-      out[M1 + COMP] = out[M1 + COMP] + dt * dm;
-      out[EN] = out[EN] + dt * de;
-      if (COMP == DIM) {
-        out[M1 + COMP] = out[M1 + COMP] + dt * dm;
-        out[EN] = out[EN] + dt * de;
-      } else {
-        // hyperdifmomsourcene5-6a: d/dx_COMP of (rho_t tau) and (tau m_DIM)
-        constexpr int FS = (COMP == 0) ? 1 : exN;  // stride across in the nu area
-        const int af = COMP == 0 ? gi : gj;
-        const HT rdf = (HT)(COMP == 0 ? T.rd0[lxo] : T.rd1[lyo]);
-        HT g7 = ((C3[nidx + FS] - C3[nidx - FS]) * rdf) * (HT)0.5;
-        HT g8 = ((C4[nidx + FS] - C4[nidx - FS]) * rdf) * (HT)0.5;
-        if ((P.bt[COMP] != 0) && zero1n(af, COMP == 0 ? n0 : n1)) { g7 = 0; g8 = 0; }
-        out[M1 + DIM] = out[M1 + DIM] + dt * (double)g7;
-        out[EN] = out[EN] + dt * (double)g8;
-      }
+}
+
+// Phase 5 along D at the tile cell r: the diffusive terms of the five passes.
+// p: the passes' ratio arrays at faces i and i-1 -- rho, e and the momentum
+// along D hold R dq, the momentum and B across D hold R.
+template <bool BG, bool MIX, bool O6, int D>
+__device__ __forceinline__ void diffuse(const char* sm, const double* chyp, int r, double k,
+                                        const typename Form<MIX>::H* p, int pn, int ps, double* out) {
+  using L = Lay<BG, MIX, O6>;
+  using HT = typename L::H;
+  constexpr int S = D == 0 ? 1 : QX;
+  constexpr int QA = D == 0 ? QV2 : QV1, QB = D == 0 ? QB2 : QB1;  // across
+  constexpr int FA = D == 0 ? M2 : M1, FD = D == 0 ? M1 : M2, FB = D == 0 ? B2 : B1;
+  const HT* const q = reinterpret_cast<const HT*>(sm + L::Q) + r;
+  HT rp, rm, mdp, mdm, map, mam;  // sums over the two cells of faces i, i-1: rho_t, m along, m across
+  if constexpr (MIX) {
+    if (BG) {
+      const double* t = reinterpret_cast<const double*>(sm + L::RT) + r;
+      rp = (HT)(t[0] + t[S]);
+      rm = (HT)(t[-S] + t[0]);
     } else {
-      // B component COMP diffused along DIM: hyperdifbsourcene (sb=-1) then
-      // hyperdifbsource (sb=+1)
-      constexpr int FS = (COMP == 0) ? 1 : exN;
-      const int af = COMP == 0 ? gi : gj;
-      const HT rdf = (HT)(COMP == 0 ? T.rd0[lxo] : T.rd1[lyo]);
-      HT g4 = ((C3[nidx + FS] - C3[nidx - FS]) * rdf) * (HT)0.5;
-      HT g6 = ((C4[nidx + FS] - C4[nidx - FS]) * rdf) * (HT)0.5;
-      if ((P.bt[COMP] != 0) && zero1n(af, COMP == 0 ? n0 : n1)) { g4 = 0; g6 = 0; }
-      out[B1 + DIM] = out[B1 + DIM] - dt * (double)g4;
-      out[EN] = out[EN] - dt * (double)g6;
-      const HT t2 = (qc + qm) * (HT)0.5, t3 = (qc + qp) * (HT)0.5;
-      const double dB = (double)((gr * nur - gl * nul) * rdl);
-      const double de = (double)((t3 * gr * nur - t2 * gl * nul) * rdl);
-      out[B1 + COMP] = out[B1 + COMP] + dt * dB;
-      out[EN] = out[EN] + dt * de;
+      rp = q[QR * QC] + q[QR * QC + S];
+      rm = q[QR * QC - S] + q[QR * QC];
     }
+    constexpr int MD = D == 0 ? QM1 : QM2, MA = D == 0 ? QM2 : QM1;
+    mdp = q[MD * QC] + q[MD * QC + S];
+    mdm = q[MD * QC - S] + q[MD * QC];
+    map = q[MA * QC] + q[MA * QC + S];
+    mam = q[MA * QC - S] + q[MA * QC];
+  } else {
+    const HT* t = BG ? reinterpret_cast<const HT*>(sm + L::RT) + r : q + QR * QC;
+    constexpr int QD = D == 0 ? QV1 : QV2;
+    const HT tm = t[-S], t0 = t[0], tp = t[S];
+    rp = t0 + tp;
+    rm = tm + t0;
+    const HT md = q[QD * QC] * t0, ma = q[QA * QC] * t0;
+    mdp = fma(q[QD * QC + S], tp, md);
+    mdm = fma(q[QD * QC - S], tm, md);
+    map = fma(q[QA * QC + S], tp, ma);
+    mam = fma(q[QA * QC - S], tm, ma);
   }
-  __syncthreads();
+  const HT va0 = q[QA * QC], b0 = q[QB * QC], bp = q[QB * QC + S], bm = q[QB * QC - S];
+  const HT vp = p[2 * pn], vm = p[2 * pn - ps];
+  const HT ap = p[3 * pn] * (q[QA * QC + S] - va0), am = p[3 * pn - ps] * (va0 - q[QA * QC - S]);
+  const HT fp = p[4 * pn] * (bp - b0), fm = p[4 * pn - ps] * (b0 - bm);
+  // the momentum pass along D counts twice (COMP == DIM); face means carry 1/2
+  const double kd = 0.5 * k * chyp[FD], ka = 0.25 * k * chyp[FA], kb = k * chyp[FB];
+  out[RHO] = fma(k * chyp[RHO], (double)(p[0] - p[-ps]), out[RHO]);
+  out[FD] = fma(kd, (double)(vp * rp - vm * rm), out[FD]);
+  out[FA] = fma(ka, (double)(ap * rp - am * rm), out[FA]);
+  out[FB] = fma(kb, (double)(fp - fm), out[FB]);
+  double e = fma(k * chyp[EN], (double)(p[pn] - p[pn - ps]), out[EN]);
+  e = fma(kd, (double)(vp * mdp - vm * mdm), e);
+  e = fma(ka, (double)(ap * map - am * mam), e);
+  out[EN] = fma(0.5 * kb, (double)(fp * (b0 + bp) - fm * (bm + b0)), e);
+}
+
+// Cross arrays along D at region cell r (hyperdifmomsourcene2-4,
+// hyperdifbsourcene1b-4): tau = (q+ - q-) (R + R-) cmax chyp / 8 of the
+// momentum across D, t: / 4 of B; rho_t tau, t, and the energy's tau m_D - t
+// B_D (two arrays in the mixed form, whose sums are double).  p: the ratios.
+template <bool BG, bool MIX, bool O6, int D>
+__device__ __forceinline__ void cross_at(const char* sm, const double* chyp, double cmax, bool zero, int r,
+                                         const typename Form<MIX>::H* p, int pn, int ps,
+                                         typename Form<MIX>::H* c, int cn) {
+  using L = Lay<BG, MIX, O6>;
+  using HT = typename L::H;
+  constexpr int S = D == 0 ? 1 : QX;
+  constexpr int QA = D == 0 ? QV2 : QV1, QB = D == 0 ? QB2 : QB1;
+  const HT* const q = reinterpret_cast<const HT*>(sm + L::Q) + r;
+  const HT kv = zero ? (HT)0 : (HT)(0.125 * cmax * chyp[D == 0 ? M2 : M1]);
+  const HT kb = zero ? (HT)0 : (HT)(0.25 * cmax * chyp[D == 0 ? B2 : B1]);
+  const HT tau = (q[QA * QC + S] - q[QA * QC - S]) * (p[3 * pn] + p[3 * pn - ps]) * kv;
+  const HT t = (q[QB * QC + S] - q[QB * QC - S]) * (p[4 * pn] + p[4 * pn - ps]) * kb;
+  const HT rt = BG ? (HT) reinterpret_cast<const double*>(sm + L::RT)[r] : q[QR * QC];
+  const HT m = MIX ? q[(D == 0 ? QM1 : QM2) * QC] : q[(D == 0 ? QV1 : QV2) * QC] * rt;
+  const HT b = q[(D == 0 ? QB1 : QB2) * QC];
+  c[0] = rt * tau;
+  c[cn] = t;
+  if constexpr (MIX) {
+    c[2 * cn] = tau * m;
+    c[3 * cn] = t * b;
+  } else {
+    c[2 * cn] = tau * m - t * b;
+  }
+}
+}  // namespace s2
+
+// The base state and the accumulator of a tile row, which its last phase
+// reads, into L2: a block's lifetime ahead of their use, two instructions per
+// thread.
+template <int MODE, bool MIX>
+__device__ __forceinline__ void prefetch_row(const KBufs& B, long nc, int x0, int gj, int n0, int n1, int tx) {
+  using ST = typename Form<MIX>::S;
+  constexpr int NL = TX * (int)sizeof(double) / 128 + 1;  // 128-byte lines a row may touch
+  if (gj > n1 - 3) return;
+  for (int k = tx; k < 12 * NL; k += TX) {
+    const int a = k / NL;
+    int gi = x0 + k % NL * 16;
+    if (gi > x0 + TX - 1) gi = x0 + TX - 1;
+    if (gi > n0 - 3) gi = n0 - 3;
+    const long c = (long)(a % 6) * nc + (long)gj * n0 + (gi < 2 ? 2 : gi);
+    const void* p = nullptr;
+    if (a < 6) {
+      if (MODE == SMAUG_INT_EULER || B.stage < 3) p = static_cast<const ST*>(B.un) + c;
+    } else if (MODE != SMAUG_INT_EULER && B.stage > 0) {
+      p = B.acc + c;
+    }
+    if (p) asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+  }
 }
 
 // Bulk tensor copy of the staged state of tile (bx, by) -- the 6 fields in
-// the storage type into s, and (gdst non-null) the 4 background fields
-// (with background fields) or rho_b alone (without) into gdst -- completing
-// on tt.bar.  Cells outside the grid read 0.  The region starts at column
-// x0 - HALO = XORG - HALO + bx TX, which the TMA-staged kernel's tile origin
-// makes a multiple of 32 cells (the copy's x offset must be 16-byte aligned).
+// the storage type into s, and (background fields) rho_b into gdst --
+// completing on tt.bar.  Cells outside the grid read 0.  The region starts at
+// column x0 - HALO = XORG - HALO + bx TX, which the TMA-staged kernel's tile
+// origin makes a multiple of 32 cells (the copy's x offset must be 16-byte
+// aligned).
 template <bool BG, bool MIX>
 __device__ __forceinline__ void tma_stage_issue(void* s, void* gdst, const TmaTile& tt, int bx, int by) {
   using ST = typename Form<MIX>::S;
-  const unsigned bytes = (s ? 6 * RC * sizeof(ST) : 0) + (gdst ? (BG ? 4 : 1) * RC * sizeof(double) : 0);
+  const unsigned bytes = 6 * RC * sizeof(ST) + (BG ? RC * sizeof(double) : 0);
   const int x = XORG - HALO + bx * TX, y = 2 - HALO + by * TY;
   fence_proxy_async_smem();
   mbar_expect_tx(tt.bar, bytes);
-  if (s) tma_load_3d(s, tt.ms, x, y, 0, tt.bar);
-  if (gdst) tma_load_3d(gdst, tt.mg, x, y, BG ? 0 : 1, tt.bar);
+  tma_load_3d(s, tt.ms, x, y, 0, tt.bar);
+  if (BG) tma_load_3d(gdst, tt.mg, x, y, 1, tt.bar);
 }
 
 // The stage for tile (bx, by) of one grid; the single-run kernels below and
-// in stage2d_tma.cu and the batched kernel (batch.cu) call it.  TMA = 1: the
-// state arrives by bulk tensor copy (tt: the block's copy schedule), and the
-// copy of the block's next tile is issued once this tile's staged arrays
-// are dead, so that it overlaps the stores.  TMA = 2 (no background
-// fields): two state buffers; the copy of the next tile's state goes to the
-// other buffer as soon as this tile's copy has arrived, so that it overlaps
-// the whole tile, and its rho_b (into 1/rho_t's array, dead by then) during
-// the stores -- two arrivals on the barrier per phase.  Returns false when a copy did
-// not complete in time (FLAG_TMA_TIMEOUT set; the block must stop).
-template <int MODE, bool BG, bool MIX, bool O6 = false, bool CG = false, int TMA = 0>
+// in stage2d_tma.cu and the batched kernel (batch_kernel.cuh) call it.  TMA:
+// the state arrives by bulk tensor copy (tt: the block's copy schedule) in
+// buffers ahead of the arrays above, and the copy of the block's next tile
+// is issued as soon as this tile's values have been derived from them.
+// Returns false when a copy did not complete in time (FLAG_TMA_TIMEOUT set;
+// the block must stop).
+template <int MODE, bool BG, bool MIX, bool O6 = false, bool CG = false, bool TMA = false>
 __device__ __forceinline__ bool stage2d_body(const KParams& P, const KBufs& B, int bx, int by,
                                              const TmaTile* tt = nullptr) {
   using ST = typename Form<MIX>::S;
+  using L = s2::Lay<BG, MIX, O6>;
+  using HT = typename L::H;
+  using s2::QC;
+  using s2::QX;
+  constexpr bool rk = MODE != SMAUG_INT_EULER;
   extern __shared__ double smem[];
-  T2<BG, MIX> T;
-  unsigned char* sp = reinterpret_cast<unsigned char*>(smem);
-  // the copy boxes land on 128-byte boundaries (the launch adds the slack);
-  // an offset added to the shared array itself, so that the compiler still
-  // addresses the tile arrays as shared memory (a pointer rebuilt from an
-  // integer would make every tile access a generic one)
-  if constexpr (TMA != 0) sp += (128u - (smem_u32(sp) & 127u)) & 127u;
-  static_assert(TMA != 2 || !BG, "double-buffered staging without background fields only");
-  T.S = reinterpret_cast<ST*>(sp);
-  sp += 6 * RC * sizeof(ST);
-  ST* const s_other = reinterpret_cast<ST*>(sp);  // TMA = 2: the second state buffer
-  if constexpr (TMA == 2) {
-    if (tt->parity) T.S = s_other;
-    sp += 6 * RC * sizeof(ST);
-  }
-  T.G = reinterpret_cast<double*>(sp);
-  sp += (BG ? 4 * RC : 0) * sizeof(double);
-  T.R = reinterpret_cast<double*>(sp);
-  T.V = T.R + RC;
-  T.dl0 = T.V + (BG ? 2 * RC : 0);
-  T.dl1 = T.dl0 + RX;
-  T.rd0 = T.dl1 + RY;
-  T.rd1 = T.rd0 + RX;
-  T.U = T.rd1 + RY;
-  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
-  T.x0 = XORG + bx * TX;
-  T.y0 = 2 + by * TY;
-  const int n0 = P.n0, n1 = P.n1;
-  // region columns x0-3 .. x0-3+RX-1 (rows y0-3 .. y0+TY+2) inside
-  // [0, n-1]: no bounds or pad checks in the staging, flux and cross-term
-  // loops
-  T.inner = bx >= 1 && by >= 1 && T.x0 - HALO + RX <= n0 && T.y0 + TY + HALO <= n1;
-  const long nc = P.ncell;
-  const ST* uin = static_cast<const ST*>(B.uin);
-
-  // ---- stage the tile, 1/rho_t, the metric -------------------------------
+  char* sm = reinterpret_cast<char*>(smem);
+  ST* raw = nullptr;
+  double* rawb = nullptr;
   if constexpr (TMA) {
-    // every thread waits on the barrier (one waiter and a block barrier
-    // measured 2.5 % slower at 4096^2)
-    void* const gdst = BG ? static_cast<void*>(T.G) : static_cast<void*>(T.R);
-    if (tt->issue_self && tid == 0) {
-      tma_stage_issue<BG, MIX>(T.S, gdst, *tt, bx, by);
-      if (TMA == 2) mbar_arrive(tt->bar);  // the phase's second arrival
-    }
+    // the copy boxes land on 128-byte boundaries (the launch adds the slack);
+    // an offset added to the shared array itself, so that the compiler still
+    // addresses the tile arrays as shared memory
+    sm += (128u - (smem_u32(sm) & 127u)) & 127u;
+    raw = reinterpret_cast<ST*>(sm);
+    rawb = reinterpret_cast<double*>(sm + 6 * RC * sizeof(ST));
+    sm += 6 * RC * sizeof(ST) + (BG ? RC * sizeof(double) : 0);
+  }
+  double* const RD0 = reinterpret_cast<double*>(sm + L::RD);
+  double* const RD1 = RD0 + RX;
+  double* const F = reinterpret_cast<double*>(sm + L::U);
+  HT* const RR = reinterpret_cast<HT*>(sm + L::U);
+  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
+  const int x0 = XORG + bx * TX, y0 = 2 + by * TY;
+  const int n0 = P.n0, n1 = P.n1;
+  const long nc = P.ncell;
+  const ST* const uin = static_cast<const ST*>(B.uin);
+  const bool hyper = P.hyperdif == 1;
+  // the region inside the grid: no source redirection in the staging
+  const bool inner = x0 - HALO >= 0 && by >= 1 && x0 - HALO + RX <= n0 && y0 + TY + HALO <= n1;
+  // running CFL maxima of the grid when the block starts
+  double seen[2];
+  {
+    const unsigned long long* cm = B.cmax_out;
+    seen[0] = __longlong_as_double(__ldcg(cm));
+    seen[1] = __longlong_as_double(__ldcg(cm + 1));
+  }
+
+  // ---- phase 0: staging ----------------------------------------------------
+  // Source cell of a region cell: the cell itself; index -1 along an axis the
+  // copy of index 5 (bc_hyperdifl); index n the stray store's source
+  // (B.padsrc); -1 for the rest (zeros).
+  auto source = [&](int gi, int gj) -> int {
+    const bool ix = gi >= 0 && gi < n0, iy = gj >= 0 && gj < n1;
+    if (ix && iy) return gj * n0 + gi;
+    if (iy) return gi == -1 ? gj * n0 + 5 : (gi == n0 ? B.padsrc[0][gj] : -1);
+    if (ix) return gj == -1 ? 5 * n0 + gi : (gj == n1 ? B.padsrc[1][gi] : -1);
+    return -1;
+  };
+  if constexpr (TMA) {
+    // every thread waits on the barrier
+    if (tt->issue_self && tid == 0) tma_stage_issue<BG, MIX>(raw, rawb, *tt, bx, by);
     const bool ok = mbar_wait(tt->bar, tt->parity, TMA_WAIT_NS);
     if (__syncthreads_or(!ok)) {
       if (tid == 0) {
@@ -430,308 +373,351 @@ __device__ __forceinline__ bool stage2d_body(const KParams& P, const KBufs& B, i
       __syncthreads();
       return false;
     }
-    if constexpr (TMA == 2) {
-      // the other buffer's last reader, the previous tile, is done
-      if (tid == 0 && tt->nbx >= 0) {
-        ST* const s0 = reinterpret_cast<ST*>(reinterpret_cast<unsigned char*>(s_other) - 6 * RC * sizeof(ST));
-        tma_stage_issue<BG, MIX>(tt->parity ? s0 : s_other, nullptr, *tt, tt->nbx, tt->nby);
-      }
-    }
-    for (int u = tid; u < RXU * RY; u += NTHREADS) {
-      const int lx = u % RXU, ly = u / RXU, r = ly * RX + lx;
-      const int gi = T.x0 - HALO + lx, gj = T.y0 - HALO + ly;
-      const bool in = T.inner || (gi >= 0 && gi < n0 && gj >= 0 && gj < n1);
-      const double rho = (double)T.S[r];  // 0 outside the grid (the copy's fill)
-      double rhob;
-      if (BG) {
-        if (!in) T.G[1 * RC + r] = 1.0;
-        rhob = T.G[1 * RC + r];
-      } else {
-        rhob = in ? T.R[r] : 1.0;
-      }
-      const double rinv = 1.0 / (rho + rhob);
-      T.R[r] = rinv;
-      if (BG) {
-        T.V[r] = (double)T.S[M1 * RC + r] * rinv;
-        T.V[RC + r] = (double)T.S[M2 * RC + r] * rinv;
-      }
-    }
-  } else {
-  for (int u = tid; u < RXU * RY; u += NTHREADS) {
-    const int lx = u % RXU, ly = u / RXU, r = ly * RX + lx;
-    const int gi = T.x0 - HALO + lx, gj = T.y0 - HALO + ly;
-    const bool in = T.inner || (gi >= 0 && gi < n0 && gj >= 0 && gj < n1);
-    const long c = (long)gj * n0 + gi;
-    double rho = 0.0, rhob = 1.0;
-#pragma unroll
-    for (int f = 0; f < 6; f++) {
-      const ST v = in ? ldin<CG>(uin + f * nc + c) : (ST)0;
-      T.S[f * RC + r] = v;
-      if (f == 0) rho = v;
-    }
-    if (BG) {
-#pragma unroll
-      for (int f = 0; f < 4; f++) {
-        const double v = in ? __ldg(B.bg + f * nc + c) : (f == 1 ? 1.0 : 0.0);
-        T.G[f * RC + r] = v;
-        if (f == 1) rhob = v;
-      }
-    } else {
-      rhob = in ? __ldg(B.bg + 1 * nc + c) : 1.0;
-      if (!in) rho = 0.0;
-    }
-    const double rinv = 1.0 / (rho + rhob);
-    T.R[r] = rinv;
-    if (BG) {
-      T.V[r] = (double)T.S[M1 * RC + r] * rinv;
-      T.V[RC + r] = (double)T.S[M2 * RC + r] * rinv;
-    }
   }
+  {
+    // all loads of a thread's region cells first, then their use
+    constexpr int NI = (RX * RY + NTHREADS - 1) / NTHREADS;
+    ST w[NI][6];
+    double rhob[NI];
+    int c[NI];
+#pragma unroll
+    for (int i = 0; i < NI; i++) {
+      const int u = tid + i * NTHREADS;
+      const int lx = u % RX, ly = u / RX;
+      const int gi = x0 - HALO + lx, gj = y0 - HALO + ly;
+      const bool in = inner || (gi >= 0 && gi < n0 && gj >= 0 && gj < n1);
+      c[i] = u >= RX * RY ? -1 : in ? gj * n0 + gi : source(gi, gj);
+      rhob[i] = 0.0;
+      if (TMA && in && u < RX * RY) {
+#pragma unroll
+        for (int f = 0; f < 6; f++) w[i][f] = raw[f * RC + u];
+        if (BG) rhob[i] = rawb[u];
+      } else {
+#pragma unroll
+        for (int f = 0; f < 6; f++) w[i][f] = c[i] >= 0 ? ldin<CG>(uin + f * nc + c[i]) : (ST)0;
+        if (BG) rhob[i] = c[i] >= 0 ? __ldg(B.bg + nc + c[i]) : 0.0;
+      }
+    }
+    prefetch_row<MODE, MIX>(B, nc, x0, y0 + ty, n0, n1, tx);
+#pragma unroll
+    for (int i = 0; i < NI; i++) {
+      const int u = tid + i * NTHREADS;
+      if (u < RX * RY) s2::derive<BG, MIX, O6>(sm, u / RX * QX + u % RX, c[i] >= 0, w[i], rhob[i]);
+    }
   }
   for (int r = tid; r < RX + RY; r += NTHREADS) {
-    if (r < RX) {
-      const int gi = T.x0 - HALO + r;
-      const double d = (gi >= 0 && gi < n0) ? B.delx[0][gi] : 1.0;
-      T.dl0[r] = d;
-      T.rd0[r] = 1.0 / d;
-    } else {
-      const int gj = T.y0 - HALO + (r - RX);
-      const double d = (gj >= 0 && gj < n1) ? B.delx[1][gj] : 1.0;
-      T.dl1[r - RX] = d;
-      T.rd1[r - RX] = 1.0 / d;
-    }
+    const int d = r < RX ? 0 : 1, g = d == 0 ? x0 - HALO + r : y0 - HALO + (r - RX);
+    RD0[r] = (g >= 0 && g < (d == 0 ? n0 : n1)) ? 1.0 / B.delx[d][g] : 1.0;
   }
 
   // ---- dt of this step and stage time ----------------------------------
   const double cin[2] = {ldsc<CG>(B.cmax_in), ldsc<CG>(B.cmax_in + 1)};
   double dt, tstage;
-  if (B.stage == 0) {
-    dt = device_dt(P, cin, ldsc<CG>(B.dt_prev), 2);
-    if (bx == 0 && by == 0 && tid == 0) {
-      *B.dt_new = dt;
-      *B.t_new = ldsc<CG>(B.t_prev) + dt;
-      B.cmax_clear[0] = B.cmax_clear[1] = B.cmax_clear[2] = 0ull;
+  {
+    const bool first = bx == 0 && by == 0 && tid == 0;
+    if (B.stage == 0) {
+      dt = device_dt(P, cin, ldsc<CG>(B.dt_prev), 2);
+      tstage = ldsc<CG>(B.t_prev);
+      if (first) {
+        *B.dt_new = dt;
+        *B.t_new = tstage + dt;
+      }
+    } else {
+      dt = ldsc<CG>(B.dt_new);
+      tstage = ldsc<CG>(B.t_prev) + (B.stage == 3 ? dt : 0.5 * dt);
     }
-    tstage = ldsc<CG>(B.t_prev);
-  } else {
-    dt = ldsc<CG>(B.dt_new);
-    tstage = ldsc<CG>(B.t_prev) + (B.stage == 3 ? dt : 0.5 * dt);
-    if (bx == 0 && by == 0 && tid == 0)
-      B.cmax_clear[0] = B.cmax_clear[1] = B.cmax_clear[2] = 0ull;
+    if (first) B.cmax_clear[0] = B.cmax_clear[1] = B.cmax_clear[2] = 0ull;
+  }
+  __syncthreads();
+  if constexpr (TMA) {
+    if (tid == 0 && tt->nbx >= 0) tma_stage_issue<BG, MIX>(raw, rawb, *tt, tt->nbx, tt->nby);
+  }
+
+  // ---- phase 1: centred fluxes -------------------------------------------
+  for (int u = tid; u < L::FXN + L::FYN; u += NTHREADS) {
+    const bool fx = u < L::FXN;
+    const int v = fx ? u : u - L::FXN;
+    const int lx = fx ? HALO - L::FH + v % L::FXW : HALO + v % TX;
+    const int ly = fx ? HALO + v / L::FXW : HALO - 2 + v / TX;
+    const int r = ly * QX + lx;
+    double g[4] = {0, 0, 0, 0}, f[5];
+    if (BG) {
+      const int gi = x0 - HALO + lx, gj = y0 - HALO + ly;
+      if (inner || (gi >= 0 && gi < n0 && gj >= 0 && gj < n1)) {
+        const long c = (long)gj * n0 + gi;
+        g[0] = __ldg(B.bg + c);
+        g[2] = __ldg(B.bg + 2 * nc + c);
+        g[3] = __ldg(B.bg + 3 * nc + c);
+      }
+    }
+    double* const o = fx ? F + v : F + 5 * L::FXN + v;
+    const int n = fx ? L::FXN : L::FYN;
+    if (fx)
+      s2::flux_at<BG, MIX, O6, 0>(sm, P.gamma, r, g, f);
+    else
+      s2::flux_at<BG, MIX, O6, 1>(sm, P.gamma, r, g, f);
+#pragma unroll
+    for (int k = 0; k < 5; k++) o[k * n] = f[k];
   }
   __syncthreads();
 
-  const int lxo = tx + HALO, lyo = ty + HALO, lo = lyo * RX + lxo;
-  const int gi = T.x0 + tx, gj = T.y0 + ty;
+  // ---- phase 2: divergence at the own cell --------------------------------
+  const int lxo = tx + HALO, lyo = ty + HALO, ro = lyo * QX + lxo;
+  const int gi = x0 + tx, gj = y0 + ty;
   const bool active = (XORG >= 2 || gi >= 2) && gi <= n0 - 3 && gj <= n1 - 3;
   const long co = active ? (long)gj * n0 + gi : 0;
-
+  const HT* const qo = reinterpret_cast<const HT*>(sm + L::Q) + ro;
+  const double rd0 = RD0[lxo], rd1 = RD1[lyo];
+  const bool z0 = (P.bt[0] != 0) && zero1n(gi, n0), z1 = (P.bt[1] != 0) && zero1n(gj, n1);
   double out[6];
-#pragma unroll
-  for (int f = 0; f < 6; f++) {
-    if (MODE != SMAUG_INT_EULER)
-      out[f] = 0.0;
-    else if (MIX)
-      out[f] = active ? base_value<MIX, CG>(B, f * nc + co) : 0.0;
-    else
-      out[f] = T.v(f, lo);
-  }
-
-  // ---- fluxes and divergence (centdiff1 / centdiff2), direction 0 then 1 --
-  constexpr int FSZ = s2::fsz<O6>();
-#pragma unroll
-  for (int d = 0; d < 2; d++) {
-    const bool o6d = O6 && d == 0;  // 6th order along dim 0 only (see s2::fsz)
-    const int fh = o6d ? 3 : 2;     // flux halo along the direction
-    const int ex = (d == 0) ? TX + 2 * fh : TX, ey = (d == 0) ? TY : TY + 2 * fh;
-    const int ox = (d == 0) ? HALO - fh : HALO, oy = (d == 0) ? HALO : HALO - fh;
-    double* F = static_cast<double*>(T.U);
-    for (int r = tid; r < ex * ey; r += NTHREADS) {
-      const int lx = ox + r % ex, ly = oy + r / ex;
-      const int ci = T.x0 - HALO + lx, cj = T.y0 - HALO + ly;
-      double f5[5] = {0, 0, 0, 0, 0};
-      if (T.inner || (ci >= 0 && ci < n0 && cj >= 0 && cj < n1)) {
-        if (d == 0)
-          flux_at<BG, MIX, 0>(T, P.gamma, ly * RX + lx, f5);
-        else
-          flux_at<BG, MIX, 1>(T, P.gamma, ly * RX + lx, f5);
-      }
-#pragma unroll
-      for (int k = 0; k < 5; k++) F[k * FSZ + r] = f5[k];
-    }
-    __syncthreads();
-    if (active) {
-      const int a = d == 0 ? gi : gj, n = d == 0 ? n0 : n1;
-      const bool z = ((P.bt[d] != 0) && zero3dn(a, n)) || (o6d && edge6(a, n));
-      const double rdl2 = 0.5 * (d == 0 ? T.rd0[lxo] : T.rd1[lyo]);
-      const int fo = (lyo - oy) * ex + (lxo - ox);
-      const int fs = d == 0 ? 1 : ex;
-      const int fld[5] = {RHO, M1, M2, EN, d == 0 ? B2 : B1};
-#pragma unroll
-      for (int k = 0; k < 5; k++) {
-        double g = o6d ? d6(F + k * FSZ, fo, fs, rdl2) : d4(F + k * FSZ, fo, fs, rdl2);
-        if (z) g = 0;
-        out[fld[k]] = out[fld[k]] - dt * g;
-      }
-      if (BG) {
-        // addenergyterms_cd2 (src/centdiff2.cu:80-115)
-        const double eb = T.v(EB, lo), bb1 = T.v(BB1, lo), bb2 = T.v(BB2, lo);
-        const double ptb = (P.gamma - 1) * eb - 0.5 * (P.gamma - 2) * (bb1 * bb1 + bb2 * bb2);
-        const double* v = T.V + d * RC;
-        double gv = o6d ? d6(v, lo, 1, rdl2) : d4(v, lo, d == 0 ? 1 : RX, rdl2);
-        if (z) gv = 0;
-        out[EN] -= dt * ptb * gv;
-        const double bbd = d == 0 ? bb1 : bb2;
-        double g0 = dflux<O6>(v, lo, 1, 0.5 * T.rd0[lxo]);
-        if (((P.bt[0] != 0) && zero3dn(gi, n0)) || (O6 && edge6(gi, n0))) g0 = 0;
-        out[EN] += dt * bb1 * bbd * g0;
-        double g1 = d4(v, lo, RX, 0.5 * T.rd1[lyo]);
-        if ((P.bt[1] != 0) && zero3dn(gj, n1)) g1 = 0;
-        out[EN] += dt * bb2 * bbd * g1;
-      }
-    }
-    __syncthreads();
-  }
-
-  // ---- gravity (addgrav_cd2, src/centdiff2.cu:118-154) --------------------
-  if (P.has_grav && active) {
-    const double rho = T.v(RHO, lo);
-    out[M1] += dt * P.g[0] * rho;
-    out[M2] += dt * P.g[1] * rho;
-    const double rr = rho * T.R[lo];
-    out[EN] += (dt * P.g[0] * T.v(M1, lo)) * rr;
-    out[EN] += (dt * P.g[1] * T.v(M2, lo)) * rr;
-  }
-
-  // ---- hyperdiffusion, in the driver's order -------------------------------
-  if (P.hyperdif == 1) {
-#define HP(K, C, D) hyper_pass<BG, MIX, K, C, D>(T, P, B, tid, active, lxo, lyo, gi, gj, dt, cin, out)
-#define SQ(K, C) stage_q2<BG, MIX, K, C, CG>(T, P, B, tid)
-    SQ(0, 0); HP(0, 0, 0); HP(0, 0, 1);
-    SQ(1, 0); HP(1, 0, 0); HP(1, 0, 1);
-    SQ(2, 0); HP(2, 0, 0); HP(2, 0, 1);
-    SQ(2, 1); HP(2, 1, 0); HP(2, 1, 1);
-    SQ(3, 1); HP(3, 1, 0);
-    SQ(3, 0); HP(3, 0, 1);
-#undef SQ
-#undef HP
-  }
-
-  // ---- user driver (source_parallel + addsourceterms2) ---------------------
-  if (P.driver == SMAUG_DRIVER_GAUSS && active) {
-    double v = P.drv_amp;
-    if (P.drv_period > 0) v *= sin(tstage * 2.0 * M_PI / P.drv_period);
-    if (P.drv_sigma[0] > 0) {
-      const double x = B.pos[0][gi] - P.drv_x0[0];
-      v *= exp(-x * x / (P.drv_sigma[0] * P.drv_sigma[0]));
-    }
-    if (P.drv_sigma[1] > 0) {
-      const double x = B.pos[1][gj] - P.drv_x0[1];
-      v *= exp(-x * x / (P.drv_sigma[1] * P.drv_sigma[1]));
-    }
-    const double rhob = BG ? T.v(RHOB, lo) : B.bg[1 * nc + co];
-    const double rr = (MODE == SMAUG_INT_EULER) ? out[RHO] : T.v(RHO, lo);
-    out[M1] = out[M1] + dt * v * (rr + rhob);
-  }
-
-  // ---- combine, write, ghost images, CFL maxima -----------------------------
-  double cm0 = P.cmax_floor[0], cm1 = P.cmax_floor[1];
-  double res[6] = {0, 0, 0, 0, 0, 0};
-  const bool is_base = (MODE == SMAUG_INT_EULER) || B.stage == 3;
   double gb[4] = {0, 0, 0, 0};  // background fields at the tile cell
-  if (active) {
-    if (MODE == SMAUG_INT_EULER) {
-#pragma unroll
-      for (int f = 0; f < 6; f++) res[f] = out[f];
-    } else {
-      const double wgt = (B.stage == 0 || B.stage == 3) ? 1.0 / 6.0 : 1.0 / 3.0;
-      const double cst = (B.stage == 2) ? 1.0 : 0.5;
-#pragma unroll
-      for (int f = 0; f < 6; f++) {
-        const double dl = out[f];
-        if (B.stage == 0) {
-          const double u = MIX ? base_value<MIX, CG>(B, f * nc + co) : T.v(f, lo);
-          B.acc[f * nc + co] = u + wgt * dl;
-          res[f] = u + cst * dl;
-        } else if (B.stage < 3) {
-          B.acc[f * nc + co] = ldsc<CG>(B.acc + f * nc + co) + wgt * dl;
-          res[f] = base_value<MIX, CG>(B, f * nc + co) + cst * dl;
-        } else {
-          res[f] = ldsc<CG>(B.acc + f * nc + co) + wgt * dl;
-        }
-      }
-    }
-    bool bad = false;
-#pragma unroll
-    for (int f = 0; f < 6; f++) bad |= !isfinite(res[f]);
-    if (bad) atomicOr(B.flags, 1);
+  {
+    const double kx = ((P.bt[0] != 0) && zero3dn(gi, n0)) || (O6 && edge6(gi, n0)) ? 0.0
+                                                                                  : dt * rd0 * (O6 ? 0.25 : 1.0 / 12.0);
+    const double ky = (P.bt[1] != 0) && zero3dn(gj, n1) ? 0.0 : dt * rd1 * (1.0 / 12.0);
+    // 12 h times the 4th-order derivative; 4 h times the 6th-order one
+    auto dx = [&](auto a) -> double {
+      const double u1 = (double)a(1) - (double)a(-1), u2 = (double)a(-2) - (double)a(2);
+      if constexpr (O6) return 3.0 * u1 + 0.6 * u2 - ((double)a(-3) - (double)a(3)) * (1.0 / 15.0);
+      return fma(8.0, u1, u2);
+    };
+    auto dy = [&](auto a) -> double {
+      return fma(8.0, (double)a(1) - (double)a(-1), (double)a(-2) - (double)a(2));
+    };
+    const double* const fx = F + ty * L::FXW + tx + L::FH;
+    const double* const fy = F + 5 * L::FXN + (ty + 2) * TX + tx;
+    auto ddx = [&](int k) { return dx([&](int s) { return fx[k * L::FXN + s]; }); };
+    auto ddy = [&](int k) { return dy([&](int s) { return fy[k * L::FYN + s * TX]; }); };
+    out[RHO] = -(kx * ddx(0)) - ky * ddy(0);
+    out[M1] = -(kx * ddx(1)) - ky * ddy(1);
+    out[M2] = -(kx * ddx(2)) - ky * ddy(2);
+    out[EN] = -(kx * ddx(3)) - ky * ddy(3);
+    out[B2] = -(kx * ddx(4));
+    out[B1] = -(ky * ddy(4));
     if (BG) {
-      gb[0] = T.v(EB, lo);
-      gb[1] = T.v(RHOB, lo);
-      gb[2] = T.v(BB1, lo);
-      gb[3] = T.v(BB2, lo);
+      if (active) {
+#pragma unroll
+        for (int f = 0; f < 4; f++) gb[f] = __ldg(B.bg + f * nc + co);
+      }
+      // addenergyterms_cd2 (src/centdiff2.cu:80-115)
+      auto vel = [&](int c, int s) -> double {
+        if constexpr (MIX)
+          return (double)qo[(s2::QM1 + c) * QC + s] * reinterpret_cast<const double*>(sm + L::RI)[ro + s];
+        else
+          return (double)qo[(s2::QV1 + c) * QC + s];
+      };
+      const double v1x = kx * dx([&](int s) { return vel(0, s); }), v2x = kx * dx([&](int s) { return vel(1, s); });
+      const double v1y = ky * dy([&](int s) { return vel(0, s * QX); });
+      const double v2y = ky * dy([&](int s) { return vel(1, s * QX); });
+      const double ptb = (P.gamma - 1) * gb[0] - 0.5 * (P.gamma - 2) * (gb[2] * gb[2] + gb[3] * gb[3]);
+      out[EN] -= ptb * (v1x + v2y);
+      out[EN] += gb[2] * (gb[2] * v1x + gb[3] * v2x) + gb[3] * (gb[2] * v1y + gb[3] * v2y);
+    }
+    if (P.has_grav) {
+      // addgrav_cd2 (src/centdiff2.cu:118-154); m rho / rho_t = v rho
+      const double rho = (double)qo[s2::QR * QC];
+      double v1, v2;
+      if constexpr (MIX) {
+        const double ri = reinterpret_cast<const double*>(sm + L::RI)[ro];
+        v1 = (double)qo[s2::QM1 * QC] * ri;
+        v2 = (double)qo[s2::QM2 * QC] * ri;
+      } else {
+        v1 = (double)qo[s2::QV1 * QC];
+        v2 = (double)qo[s2::QV2 * QC];
+      }
+      out[M1] += dt * P.g[0] * rho;
+      out[M2] += dt * P.g[1] * rho;
+      out[EN] += dt * (P.g[0] * v1 + P.g[1] * v2) * rho;
     }
   }
-  if constexpr (TMA != 0) {
-    // the staged arrays are dead: copy the block's next tile (TMA = 2: its
-    // rho_b) during the stores
+
+  // base state and accumulator of the own cell, all loaded before the first
+  // store (a load after a store to the accumulator would wait for its own
+  // round trip) and before the last phase's arithmetic
+  double ub[6], ac[6];
+  auto load_base = [&] {
+    if (!active) return;
+    if (!rk || B.stage < 3) {
+#pragma unroll
+      for (int f = 0; f < 6; f++) ub[f] = base_value<MIX, CG>(B, f * nc + co);
+    }
+    if (rk && B.stage > 0) {
+#pragma unroll
+      for (int f = 0; f < 6; f++) ac[f] = ldsc<CG>(B.acc + f * nc + co);
+    }
+  };
+  if (!hyper) {
+    load_base();
+  } else {
     __syncthreads();
-    if (tid == 0 && tt->nbx >= 0)
-      tma_stage_issue<BG, MIX>(TMA == 2 ? nullptr : static_cast<void*>(T.S),
-                               BG ? static_cast<void*>(T.G) : static_cast<void*>(T.R), *tt, tt->nbx, tt->nby);
-  }
-  if (active) {
-    int ix[3], iy[3];
-    ix[0] = gi;
-    iy[0] = gj;
-    const int nx = 1 + ghost_images(gi, n0, P.bc[0], ix + 1);
-    const int ny = 1 + ghost_images(gj, n1, P.bc[1], iy + 1);
-    bool negated = false;  // res holds the negated values
-    for (int b = 0; b < ny; b++)
-      for (int a2 = 0; a2 < nx; a2++) {
-        const long cc = (long)iy[b] * n0 + ix[a2];
-        // antisymmetric images carry the opposite sign (negation is exact)
-        const bool neg = ((a2 > 0) && P.gneg[0]) != ((b > 0) && P.gneg[1]);
-        if (neg != negated) {
-#pragma unroll
-          for (int f = 0; f < 6; f++) res[f] = -res[f];
-          negated = neg;
-        }
-        const double* r = res;
-#pragma unroll
-        for (int f = 0; f < 6; f++) store_value<MIX>(B, f * nc + cc, r[f], is_base);
-        double eb, rb, b1b, b2b;
-        if (BG && a2 == 0 && b == 0) {
-          eb = gb[0]; rb = gb[1]; b1b = gb[2]; b2b = gb[3];
-        } else {
-          eb = B.bg[0 * nc + cc]; rb = B.bg[1 * nc + cc]; b1b = B.bg[2 * nc + cc]; b2b = B.bg[3 * nc + cc];
-        }
-        double c0, c1;
-        cfast2_both(P.gamma, r[RHO], r[M1], r[M2], r[EN], r[B1], r[B2], eb, rb, b1b, b2b, c0, c1);
-        cm0 = dmax0(cm0, c0);
-        cm1 = dmax0(cm1, c1);
+    // ---- phase 3: nu ratios ------------------------------------------------
+    // pieces of rows: 11 faces (three to a 32-cell row), 9 for a 16-cell one
+    constexpr int NS = (TX + 11) / 11, SL = (TX + NS) / NS;
+    constexpr int NXT = (3 * TY + 2 * (TY + 2)) * NS, NYT = 3 * TX + 2 * (TX + 2);
+    for (int u = tid; u < NXT + NYT; u += NTHREADS) {
+      if (u < NXT) {
+        // rows of rho, e, v1 on the tile, of v2, b2 one more on each side
+        const int s = u % NS, v = u / NS;
+        const bool cr = v >= 3 * TY;
+        const int k = cr ? 3 + (v - 3 * TY) / (TY + 2) : v / TY;
+        const int row = cr ? (v - 3 * TY) % (TY + 2) : 1 + v % TY;  // 0 .. TY+1
+        const int fld = k == 0 ? s2::QR : k == 1 ? s2::QE : k == 2 ? s2::QV1 : k == 3 ? s2::QV2 : s2::QB2;
+        const int f0 = s * SL, n = TX + 1 - f0 < SL ? TX + 1 - f0 : SL;
+        const HT* q = reinterpret_cast<const HT*>(sm + L::Q) + fld * QC + (row + HALO - 1) * QX + HALO - 1 + f0;
+        HT* o = RR + k * L::RXN + row * L::RXW + f0;
+        s2::ratio_line<SL, 1, (TX + 1) % SL == 0>(q, n, [&](int i, HT r, HT dq) { o[i] = cr ? r : r * dq; });
+      } else {
+        // columns of rho, e, v2 on the tile, of v1, b1 one more on each side
+        const int v = u - NXT;
+        const bool cr = v >= 3 * TX;
+        const int k = cr ? 3 + (v - 3 * TX) / (TX + 2) : v / TX;
+        const int col = cr ? (v - 3 * TX) % (TX + 2) : 1 + v % TX;  // 0 .. TX+1
+        const int fld = k == 0 ? s2::QR : k == 1 ? s2::QE : k == 2 ? s2::QV2 : k == 3 ? s2::QV1 : s2::QB1;
+        const HT* q = reinterpret_cast<const HT*>(sm + L::Q) + fld * QC + (HALO - 1) * QX + col + HALO - 1;
+        HT* o = RR + 5 * L::RXN + k * L::RYN + col;
+        s2::ratio_line<TY + 1, QX, true>(q, TY + 1, [&](int i, HT r, HT dq) { o[i * L::RYW] = cr ? r : r * dq; });
       }
+    }
+    __syncthreads();
+    // ---- phase 4: cross arrays (zero outside [2, n-3] and next to the edges) -
+    HT* const CX = RR + 5 * (L::RXN + L::RYN);
+    HT* const CY = CX + L::NC * L::CXN;
+    for (int u = tid; u < L::CXN + L::CYN; u += NTHREADS) {
+      const bool xd = u < L::CXN;
+      const int v = xd ? u : u - L::CXN;
+      const int cx = xd ? v % TX + 1 : v % L::CYW, cy = xd ? v / TX : v / L::CYW + 1;  // tile cell + 1
+      const int ci = x0 - 1 + cx, cj = y0 - 1 + cy;
+      const int r = (cy + HALO - 1) * QX + cx + HALO - 1;
+      const bool out2 = ci < 2 || ci > n0 - 3 || cj < 2 || cj > n1 - 3;
+      if (xd)
+        s2::cross_at<BG, MIX, O6, 0>(sm, P.chyp, cin[0], out2 || ((P.bt[0] != 0) && zero1n(ci, n0)), r,
+                                     RR + cy * L::RXW + cx, L::RXN, 1, CX + v, L::CXN);
+      else
+        s2::cross_at<BG, MIX, O6, 1>(sm, P.chyp, cin[1], out2 || ((P.bt[1] != 0) && zero1n(cj, n1)), r,
+                                     RR + 5 * L::RXN + cy * L::RYW + cx, L::RYN, L::RYW, CY + v, L::CYN);
+    }
+    __syncthreads();
+    // ---- phase 5: diffusive and cross terms ----------------------------------
+    load_base();
+    s2::diffuse<BG, MIX, O6, 0>(sm, P.chyp, ro, z0 ? 0.0 : dt * cin[0] * rd0, RR + (ty + 1) * L::RXW + tx + 1,
+                                L::RXN, 1, out);
+    s2::diffuse<BG, MIX, O6, 1>(sm, P.chyp, ro, z1 ? 0.0 : dt * cin[1] * rd1,
+                                RR + 5 * L::RXN + (ty + 1) * L::RYW + tx + 1, L::RYN, L::RYW, out);
+    {
+      // d/dy of the x passes' arrays, d/dx of the y passes'
+      const double ky = z1 ? 0.0 : 0.5 * dt * rd1, kx = z0 ? 0.0 : 0.5 * dt * rd0;
+      const HT* const c = CX + (ty + 1) * TX + tx;
+      auto dc = [&](int k) -> double { return (double)(c[k * L::CXN + TX] - c[k * L::CXN - TX]); };
+      out[M1] = fma(ky, dc(0), out[M1]);
+      out[B1] = fma(-ky, dc(1), out[B1]);
+      out[EN] = fma(ky, dc(2), out[EN]);
+      if constexpr (MIX) out[EN] = fma(-ky, dc(3), out[EN]);
+      const HT* const d = CY + ty * L::CYW + tx + 1;
+      auto dd = [&](int k) -> double { return (double)(d[k * L::CYN + 1] - d[k * L::CYN - 1]); };
+      out[M2] = fma(kx, dd(0), out[M2]);
+      out[B2] = fma(-kx, dd(1), out[B2]);
+      out[EN] = fma(kx, dd(2), out[EN]);
+      if constexpr (MIX) out[EN] = fma(-kx, dd(3), out[EN]);
+    }
   }
-  __shared__ double red[NTHREADS / 32][2];
-  for (int o = 16; o > 0; o >>= 1) {
-    cm0 = dmax0(cm0, __shfl_xor_sync(0xffffffffu, cm0, o));
-    cm1 = dmax0(cm1, __shfl_xor_sync(0xffffffffu, cm1, o));
+
+  // ---- driver, stage sum, stores, ghost images, CFL maxima ------------------
+  double cm[2] = {seen[0], seen[1]};
+  if (P.cmax_floor[0] > cm[0]) cm[0] = P.cmax_floor[0];
+  if (P.cmax_floor[1] > cm[1]) cm[1] = P.cmax_floor[1];
+  if (active) {
+    double res[6];
+    const bool is_base = !rk || B.stage == 3;
+    const double wgt = (B.stage == 0 || B.stage == 3) ? 1.0 / 6.0 : 1.0 / 3.0;
+    const double cst = (B.stage == 2) ? 1.0 : 0.5;
+    if (P.driver == SMAUG_DRIVER_GAUSS) {
+      // source_parallel + addsourceterms2
+      double v = P.drv_amp;
+      if (P.drv_period > 0) v *= sin(tstage * 2.0 * M_PI / P.drv_period);
+      if (P.drv_sigma[0] > 0) {
+        const double x = B.pos[0][gi] - P.drv_x0[0];
+        v *= exp(-x * x / (P.drv_sigma[0] * P.drv_sigma[0]));
+      }
+      if (P.drv_sigma[1] > 0) {
+        const double x = B.pos[1][gj] - P.drv_x0[1];
+        v *= exp(-x * x / (P.drv_sigma[1] * P.drv_sigma[1]));
+      }
+      const double rr = rk ? (double)qo[s2::QR * QC] : ub[RHO] + out[RHO];
+      out[M1] = out[M1] + dt * v * (rr + gb[1]);
+    }
+#pragma unroll
+    for (int f = 0; f < 6; f++) {
+      if (!rk) {
+        res[f] = ub[f] + out[f];
+      } else if (B.stage == 3) {
+        res[f] = ac[f] + wgt * out[f];
+      } else {
+        B.acc[f * nc + co] = (B.stage == 0 ? ub[f] : ac[f]) + wgt * out[f];
+        res[f] = ub[f] + cst * out[f];
+      }
+    }
+    int hmax = 0;  // largest exponent word: infinities and NaN have 0x7ff
+#pragma unroll
+    for (int f = 0; f < 6; f++) hmax = max(hmax, __double2hiint(res[f]) & 0x7fffffff);
+    if (hmax >= 0x7ff00000) atomicOr(B.flags, 1);
+    auto speeds = [&](const double* g) {
+      if (may_exceed<2, BG>(P.gamma, res, g, cm)) {
+        const double2 c =
+            cfast2_call(P.gamma, res[RHO], res[M1], res[M2], res[EN], res[B1], res[B2], g[0], g[1], g[2], g[3]);
+        cm[0] = dmax0(cm[0], c.x);
+        cm[1] = dmax0(cm[1], c.y);
+      }
+    };
+#pragma unroll
+    for (int f = 0; f < 6; f++) store_value<MIX>(B, f * nc + co, res[f], is_base);
+    speeds(gb);
+    // tiles that hold cells within 4 of an end of the interior have images
+    if (x0 < 6 || y0 < 6 || x0 + TX > n0 - 6 || y0 + TY > n1 - 6) {
+      int ix[3], iy[3];
+      ix[0] = gi;
+      iy[0] = gj;
+      const int nx = 1 + ghost_images(gi, n0, P.bc[0], ix + 1);
+      const int ny = 1 + ghost_images(gj, n1, P.bc[1], iy + 1);
+      bool negated = false;  // res holds the negated values
+      for (int b = 0; b < ny; b++)
+        for (int a = b == 0 ? 1 : 0; a < nx; a++) {
+          const long cc = (long)iy[b] * n0 + ix[a];
+          // antisymmetric images carry the opposite sign (negation is exact)
+          const bool neg = ((a > 0) && P.gneg[0]) != ((b > 0) && P.gneg[1]);
+          if (neg != negated) {
+#pragma unroll
+            for (int f = 0; f < 6; f++) res[f] = -res[f];
+            negated = neg;
+          }
+#pragma unroll
+          for (int f = 0; f < 6; f++) store_value<MIX>(B, f * nc + cc, res[f], is_base);
+          // without background fields an image has its source's fast speeds
+          // unless its sign changed
+          if (BG || neg) {
+            double g[4] = {0, 0, 0, 0};
+            if (BG) {
+#pragma unroll
+              for (int f = 0; f < 4; f++) g[f] = __ldg(B.bg + f * nc + cc);
+            }
+            speeds(g);
+          }
+        }
+    }
   }
-  if ((tid & 31) == 0) {
-    red[tid >> 5][0] = cm0;
-    red[tid >> 5][1] = cm1;
-  }
-  __syncthreads();
-  if (tid < 2) {
-    double v = 0.0;
-    for (int w = 0; w < NTHREADS / 32; w++) v = dmax0(v, red[w][tid]);
-    atomicMax(&B.cmax_out[tid], (unsigned long long)__double_as_longlong(v));
+  // maxima above what the grid had when the block started
+  if (__any_sync(0xffffffffu, cm[0] > seen[0] || cm[1] > seen[1])) {
+#pragma unroll
+    for (int d = 0; d < 2; d++) {
+      for (int o = 16; o > 0; o >>= 1) cm[d] = dmax0(cm[d], __shfl_xor_sync(0xffffffffu, cm[d], o));
+      if ((tid & 31) == 0) atomicMax(&B.cmax_out[d], (unsigned long long)__double_as_longlong(cm[d]));
+    }
   }
   return true;
 }
 
 template <int MODE, bool BG, bool MIX, bool O6>
-__global__ void __launch_bounds__(NTHREADS, SMAUG_MINB2D) stage2d_fast(const KParams P, const KBufs B) {
+__global__ void __launch_bounds__(NTHREADS, MIX ? SMAUG_MINB2D_MIX : SMAUG_MINB2D)
+    stage2d_fast(const KParams P, const KBufs B) {
   stage2d_body<MODE, BG, MIX, O6>(P, B, blockIdx.x, blockIdx.y);
 }
 

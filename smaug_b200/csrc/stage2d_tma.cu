@@ -10,16 +10,12 @@
 // 16-byte aligned).  Tile column 0 holds only the interior column x = 2.
 //
 // One thread issues the copies of a tile -- the 6 fields of the stage input
-// as one box [6][14][40], and the 4 background fields (or rho_b alone) as a
-// second box -- completing on the block's mbarrier.  Two launch forms: one
-// block per tile, or a persistent grid (resident blocks per SM x SMs; block
-// b owns the tiles b, b + grid, ...).  In the persistent form a block copies
-// its next tile as soon as the current tile's staged arrays are dead (after
-// the last hyperdiffusion pass and the reads of its combine), overlapping
-// the copy with the tile's stores, ghost images and CFL epilogue; the mixed
-// form without background fields, where a second state buffer still fits 4
-// blocks per SM, copies the next tile's state into the other buffer a whole
-// tile ahead and its rho_b during the stores (two arrivals per phase).
+// as one box [6][14][40] and, with background fields, rho_b as a second box --
+// into buffers ahead of the body's arrays, completing on the block's mbarrier.
+// Two launch forms: one block per tile, or a persistent grid (resident blocks
+// per SM x SMs; block b owns the tiles b, b + grid, ...).  In the persistent
+// form a block copies its next tile as soon as the current tile's values have
+// been derived from the buffers, overlapping the copy with the rest of the tile.
 // Cells outside the grid read 0 (the copy's fill value), as the per-thread
 // staging stores them.  Every wait on the mbarrier is bounded (TMA_WAIT_NS);
 // a block whose copy does not arrive sets FLAG_TMA_TIMEOUT, waits (bounded)
@@ -40,8 +36,6 @@ constexpr int TX = 32, TY = 8;
 constexpr int RX = TX + 8;  // 3 + 32 + 5 columns: 16-byte-multiple rows in float and double
 constexpr int RY = TY + 2 * HALO;
 constexpr int RC = RX * RY;
-constexpr int RXU = RX;  // all 40 columns (the last two are never read; skipping them in the
-                        // region loops measured more shared-memory bank conflicts)
 constexpr int NTHREADS = TX * TY;
 constexpr int XORG = 3 - TX;  // tile column bx starts at 3 + TX (bx - 1)
 static_assert((XORG - HALO) % 32 == 0, "region start must be a multiple of 32 cells");
@@ -49,21 +43,12 @@ static_assert(RX * sizeof(float) % 16 == 0 && RX * sizeof(double) % 16 == 0, "ro
 
 #include "stage2d.cuh"
 
-// the staging of a specialisation: two state buffers where they keep 4
-// blocks per SM (the mixed form without background fields), else one
-template <bool BG, bool MIX>
-__host__ __device__ constexpr int tma_form() {
-  return (!BG && MIX) ? 2 : 1;
-}
-
 template <int MODE, bool BG, bool MIX>
-__global__ void __launch_bounds__(NTHREADS, SMAUG_MINB2D)
+__global__ void __launch_bounds__(NTHREADS, 2)
     stage2d_tma_kernel(const KParams P, const KBufs B, const __grid_constant__ CUtensorMap ms,
                        const __grid_constant__ CUtensorMap mg, int nbx, int ntiles) {
   __shared__ unsigned long long bar;
-  // arrivals per phase: the copy of the state and, with two state buffers,
-  // the separate copy of rho_b
-  if (threadIdx.x == 0 && threadIdx.y == 0) mbar_init(&bar, tma_form<BG, MIX>());
+  if (threadIdx.x == 0 && threadIdx.y == 0) mbar_init(&bar, 1);
   __syncthreads();
   TmaTile tt{&ms, &mg, &bar, 0u, true, -1, 0};
   unsigned k = 0;
@@ -73,17 +58,17 @@ __global__ void __launch_bounds__(NTHREADS, SMAUG_MINB2D)
     tt.issue_self = k == 0;
     tt.nbx = next < ntiles ? next % nbx : -1;
     tt.nby = next / nbx;
-    if (!stage2d_body<MODE, BG, MIX, false, false, tma_form<BG, MIX>()>(P, B, tile % nbx, tile / nbx, &tt))
-      return;
+    if (!stage2d_body<MODE, BG, MIX, false, false, true>(P, B, tile % nbx, tile / nbx, &tt)) return;
   }
 }
 
-// dynamic shared memory: the stage body's layout plus alignment slack (the
-// body rounds its base up to 128 bytes for the copies)
+// dynamic shared memory: the stage body's layout behind the copy buffers,
+// plus alignment slack (the body rounds its base up to 128 bytes for the
+// copies)
 template <bool BG, bool MIX>
 constexpr size_t tma_smem() {
-  return s2::smem_bytes<BG, MIX, false>() + 128 +
-         (tma_form<BG, MIX>() == 2 ? 6 * RC * sizeof(typename Form<MIX>::S) : 0);
+  return s2::smem_bytes<BG, MIX, false>() + 128 + 6 * RC * sizeof(typename Form<MIX>::S) +
+         (BG ? RC * sizeof(double) : 0);
 }
 
 template <int MODE, bool BG, bool MIX>
