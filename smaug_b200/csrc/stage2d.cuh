@@ -29,11 +29,12 @@
 //   1  centred fluxes of both directions on the tile +-2
 //   2  own cell: divergence of the fluxes, background coupling, gravity
 //   3  nu ratios of all ten passes; one thread takes a line of a field (11
-//      faces along x, the tile's height along y) through running windows
-//      (RatioWindow): 14 to 16 loads per line instead of six per face
-//   4  cross-term arrays of the four passes that have them
-//   5  own cell: diffusive and cross terms, driver, stage sum, stores, ghost
-//      images, CFL maxima
+//      faces along x, the tile's height along y; ratio_line): 14 to 16 loads
+//      per line instead of six per face
+//   4  own cell: diffusive terms; cross-term arrays of the four passes that
+//      have them
+//   5  own cell: cross terms, driver, stage sum, stores, ghost images, CFL
+//      maxima
 // The arrays of phases 1-2 and 3-5 share their memory.
 #pragma once
 
@@ -88,9 +89,9 @@ __device__ __forceinline__ void derive(char* sm, int r, bool ok, const ST* w, do
   double rt = BG ? (double)w[RHO] + rhob : (double)w[RHO];
   if (!ok) rt = 1.0;
   const double ri = recip(rt);
-  const double v1 = m1 * ri, v2 = m2 * ri;
+  const double v1 = mulr(m1, ri), v2 = mulr(m2, ri);
   Q[QR * QC + r] = (HT)w[RHO];
-  Q[QE * QC + r] = (HT)((double)w[EN] - 0.5 * ((b1 * b1 + b2 * b2) + (m1 * v1 + m2 * v2)));
+  Q[QE * QC + r] = (HT)fma(-0.5, fma(b1, b1, fma(b2, b2, fma(m1, v1, mulr(m2, v2)))), (double)w[EN]);
   Q[QV1 * QC + r] = (HT)v1;
   Q[QV2 * QC + r] = (HT)v2;
   Q[QB1 * QC + r] = (HT)w[B1];
@@ -104,77 +105,69 @@ __device__ __forceinline__ void derive(char* sm, int r, bool ok, const ST* w, do
   if (BG) reinterpret_cast<double*>(sm + L::RT)[r] = rt;
 }
 
-// fluxes along D of rho, m1, m2, e and the B component across D at region
-// cell r (src/centdiff1.cu:51-197, src/centdiff2.cu:203-323):
+// fluxes of rho, m1, m2, e and the B component across at region cell r, along
+// dim 0 (X) into fx[k * sx] and along dim 1 (Y) into fy[k * sy]
+// (src/centdiff1.cu:51-197, src/centdiff2.cu:203-323):
 //   F_rho = m_D (= m_D rho'/rho_t + rho_b m_D/rho_t)
 //   F_m_c = v_D m_c + delta_cD p_t - (B'_c Bb_D + Bb_c B'_D) - B'_c B'_D
 //   F_e   = v_D (e + p_t + e_b) - (B'_D (Bb.m) + Bb_D (B'.m) + B'_D (B'.m)) / rho_t
 //   F_B_c = v_D (B'_c + Bb_c) - v_c (B'_D + Bb_D)
+// The momentum flux across is symmetric and the induction flux antisymmetric.
 // In the FP64 form e and p_t come from the staged q_e = e - (B'^2 + m.v)/2:
 // p_t = (g-1)(q_e + B'^2/2) - (g-2)(B'.Bb + B'^2/2).
-template <bool BG, bool MIX, bool O6, int D>
-__device__ __forceinline__ void flux_at(const char* sm, double gamma, int r, const double* g, double* F) {
+template <bool BG, bool MIX, bool O6, bool X, bool Y>
+__device__ __forceinline__ void flux_at(const char* sm, double gamma, int r, const double* g, double* fx, int sx,
+                                        double* fy, int sy) {
   using L = Lay<BG, MIX, O6>;
   using HT = typename L::H;
   const HT* const Q = reinterpret_cast<const HT*>(sm + L::Q);
   const double b1 = (double)Q[QB1 * QC + r], b2 = (double)Q[QB2 * QC + r];
   double m1, m2, v1, v2, e, msr;
-  const double hb = 0.5 * (b1 * b1 + b2 * b2);
+  const double hb = 0.5 * fma(b1, b1, mulr(b2, b2));
   if constexpr (MIX) {
     const double ri = reinterpret_cast<const double*>(sm + L::RI)[r];
     m1 = (double)Q[QM1 * QC + r];
     m2 = (double)Q[QM2 * QC + r];
-    v1 = m1 * ri;
-    v2 = m2 * ri;
-    msr = 0.5 * (m1 * v1 + m2 * v2);
+    v1 = mulr(m1, ri);
+    v2 = mulr(m2, ri);
+    msr = 0.5 * fma(m1, v1, mulr(m2, v2));
     e = (double)Q[QEN * QC + r] - msr;
   } else {
     const double rt = BG ? reinterpret_cast<const double*>(sm + L::RT)[r] : (double)Q[QR * QC + r];
     v1 = (double)Q[QV1 * QC + r];
     v2 = (double)Q[QV2 * QC + r];
-    m1 = v1 * rt;
-    m2 = v2 * rt;
-    msr = 0.5 * (m1 * v1 + m2 * v2);
+    m1 = mulr(v1, rt);
+    m2 = mulr(v2, rt);
+    msr = 0.5 * fma(m1, v1, mulr(m2, v2));
     e = (double)Q[QE * QC + r] + hb;
   }
   const double bb1 = BG ? g[2] : 0.0, bb2 = BG ? g[3] : 0.0;
   // computept3 (src/dervfields.cu:107-153); e holds the energy without m.v/2
-  const double pt = (gamma - 1.0) * e - (gamma - 2.0) * (BG ? (b1 * bb1 + b2 * bb2) + hb : hb);
-  const double md = D == 0 ? m1 : m2, vd = D == 0 ? v1 : v2, bd = D == 0 ? b1 : b2;
-  const double bbd = D == 0 ? bb1 : bb2;
-  const double t1 = BG ? b1 + bb1 : b1, t2 = BG ? b2 + bb2 : b2, td = D == 0 ? t1 : t2;
-  const double bv = b1 * v1 + b2 * v2;
-  const double tv = BG ? bv + (bb1 * v1 + bb2 * v2) : bv;  // (B' + B_b) . v
-  F[0] = md;
-  F[1] = vd * m1 + (D == 0 ? pt : 0.0) - (BG ? b1 * td + bb1 * bd : b1 * bd);
-  F[2] = vd * m2 + (D == 1 ? pt : 0.0) - (BG ? b2 * td + bb2 * bd : b2 * bd);
-  F[3] = vd * ((e + msr) + pt + (BG ? g[0] : 0.0)) - (BG ? bd * tv + bbd * bv : bd * bv);
-  F[4] = D == 0 ? v1 * t2 - v2 * t1 : v2 * t1 - v1 * t2;
-}
-
-// N faces of a line of q, stride S: the ratios of faces l0 .. l0+N-1 from q(l0-2
-// .. l0+N+2); put(k, R, q(l+1) - q(l)) takes face l0 + k.  Faces from n on are
-// left out (the last piece of a row may be shorter).
-template <int N, int S, bool FULL, typename H, typename Put>
-__device__ __forceinline__ void ratio_line(const H* q, int n, Put put) {
-  RatioWindow<H> w{};
-  H a1 = 0, a2 = 0, a3 = 0;  // q one, two and three cells back
-#pragma unroll
-  for (int k = 0; k < N + 5; k++) {
-    if (FULL || k < n + 5) {
-      const H a = q[(k - 2) * S];
-      H t5 = 0, t4 = 0;
-      if (k >= 1) w.d1(a, a1, t5);
-      if (k >= 3) w.d3(a, a1, a2, a3, t4);
-      if (k >= 5) put(k - 5, nu_ratio(t4, t5), a2 - a3);
-      a3 = a2;
-      a2 = a1;
-      a1 = a;
-    }
+  const double pt =
+      fma(gamma - 1.0, e, -mulr(gamma - 2.0, BG ? fma(b1, bb1, fma(b2, bb2, hb)) : hb));
+  const double t1 = BG ? b1 + bb1 : b1, t2 = BG ? b2 + bb2 : b2;
+  const double bv = fma(b1, v1, mulr(b2, v2));
+  const double tv = BG ? fma(bb1, v1, fma(bb2, v2, bv)) : bv;  // (B' + B_b) . v
+  const double h = (e + msr) + (BG ? pt + g[0] : pt);
+  const double s12 = fma(v1, m2, -(BG ? fma(b1, t2, mulr(bb1, b2)) : mulr(b1, b2)));
+  const double ind = fma(v1, t2, -mulr(v2, t1));
+  if (X) {
+    fx[0] = m1;
+    fx[sx] = fma(v1, m1, pt) - (BG ? fma(b1, t1, mulr(bb1, b1)) : mulr(b1, b1));
+    fx[2 * sx] = s12;
+    fx[3 * sx] = fma(v1, h, -(BG ? fma(b1, tv, mulr(bb1, bv)) : mulr(b1, bv)));
+    fx[4 * sx] = ind;
+  }
+  if (Y) {
+    fy[0] = m2;
+    fy[sy] = s12;
+    fy[2 * sy] = fma(v2, m2, pt) - (BG ? fma(b2, t2, mulr(bb2, b2)) : mulr(b2, b2));
+    fy[3 * sy] = fma(v2, h, -(BG ? fma(b2, tv, mulr(bb2, bv)) : mulr(b2, bv)));
+    fy[4 * sy] = -ind;
   }
 }
 
-// Phase 5 along D at the tile cell r: the diffusive terms of the five passes.
+// The diffusive terms of the five passes along D at the tile cell r.
 // p: the passes' ratio arrays at faces i and i-1 -- rho, e and the momentum
 // along D hold R dq, the momentum and B across D hold R.
 template <bool BG, bool MIX, bool O6, int D>
@@ -207,7 +200,7 @@ __device__ __forceinline__ void diffuse(const char* sm, const double* chyp, int 
     const HT tm = t[-S], t0 = t[0], tp = t[S];
     rp = t0 + tp;
     rm = tm + t0;
-    const HT md = q[QD * QC] * t0, ma = q[QA * QC] * t0;
+    const HT md = mulr(q[QD * QC], t0), ma = mulr(q[QA * QC], t0);
     mdp = fma(q[QD * QC + S], tp, md);
     mdm = fma(q[QD * QC - S], tm, md);
     map = fma(q[QA * QC + S], tp, ma);
@@ -215,18 +208,18 @@ __device__ __forceinline__ void diffuse(const char* sm, const double* chyp, int 
   }
   const HT va0 = q[QA * QC], b0 = q[QB * QC], bp = q[QB * QC + S], bm = q[QB * QC - S];
   const HT vp = p[2 * pn], vm = p[2 * pn - ps];
-  const HT ap = p[3 * pn] * (q[QA * QC + S] - va0), am = p[3 * pn - ps] * (va0 - q[QA * QC - S]);
-  const HT fp = p[4 * pn] * (bp - b0), fm = p[4 * pn - ps] * (b0 - bm);
+  const HT ap = mulr(p[3 * pn], q[QA * QC + S] - va0), am = mulr(p[3 * pn - ps], va0 - q[QA * QC - S]);
+  const HT fp = mulr(p[4 * pn], bp - b0), fm = mulr(p[4 * pn - ps], b0 - bm);
   // the momentum pass along D counts twice (COMP == DIM); face means carry 1/2
   const double kd = 0.5 * k * chyp[FD], ka = 0.25 * k * chyp[FA], kb = k * chyp[FB];
   out[RHO] = fma(k * chyp[RHO], (double)(p[0] - p[-ps]), out[RHO]);
-  out[FD] = fma(kd, (double)(vp * rp - vm * rm), out[FD]);
-  out[FA] = fma(ka, (double)(ap * rp - am * rm), out[FA]);
+  out[FD] = fma(kd, (double)fma(vp, rp, -mulr(vm, rm)), out[FD]);
+  out[FA] = fma(ka, (double)fma(ap, rp, -mulr(am, rm)), out[FA]);
   out[FB] = fma(kb, (double)(fp - fm), out[FB]);
   double e = fma(k * chyp[EN], (double)(p[pn] - p[pn - ps]), out[EN]);
-  e = fma(kd, (double)(vp * mdp - vm * mdm), e);
-  e = fma(ka, (double)(ap * map - am * mam), e);
-  out[EN] = fma(0.5 * kb, (double)(fp * (b0 + bp) - fm * (bm + b0)), e);
+  e = fma(kd, (double)fma(vp, mdp, -mulr(vm, mdm)), e);
+  e = fma(ka, (double)fma(ap, map, -mulr(am, mam)), e);
+  out[EN] = fma(0.5 * kb, (double)fma(fp, b0 + bp, -mulr(fm, bm + b0)), e);
 }
 
 // Cross arrays along D at region cell r (hyperdifmomsourcene2-4,
@@ -255,32 +248,28 @@ __device__ __forceinline__ void cross_at(const char* sm, const double* chyp, dou
     c[2 * cn] = tau * m;
     c[3 * cn] = t * b;
   } else {
-    c[2 * cn] = tau * m - t * b;
+    c[2 * cn] = fma(tau, m, -mulr(t, b));
   }
 }
 }  // namespace s2
 
 // The base state and the accumulator of a tile row, which its last phase
-// reads, into L2: a block's lifetime ahead of their use, two instructions per
-// thread.
+// reads, into L2, a block's lifetime ahead of their use: lane k of the row
+// takes field k of the twelve.
 template <int MODE, bool MIX>
 __device__ __forceinline__ void prefetch_row(const KBufs& B, long nc, int x0, int gj, int n0, int n1, int tx) {
   using ST = typename Form<MIX>::S;
-  constexpr int NL = TX * (int)sizeof(double) / 128 + 1;  // 128-byte lines a row may touch
-  if (gj > n1 - 3) return;
-  for (int k = tx; k < 12 * NL; k += TX) {
-    const int a = k / NL;
-    int gi = x0 + k % NL * 16;
-    if (gi > x0 + TX - 1) gi = x0 + TX - 1;
-    if (gi > n0 - 3) gi = n0 - 3;
-    const long c = (long)(a % 6) * nc + (long)gj * n0 + (gi < 2 ? 2 : gi);
-    const void* p = nullptr;
-    if (a < 6) {
-      if (MODE == SMAUG_INT_EULER || B.stage < 3) p = static_cast<const ST*>(B.un) + c;
-    } else if (MODE != SMAUG_INT_EULER && B.stage > 0) {
-      p = B.acc + c;
-    }
-    if (p) asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+  if (tx >= 12 || gj > n1 - 3) return;
+  const bool base = tx < 6;
+  if (base ? !(MODE == SMAUG_INT_EULER || B.stage < 3) : !(MODE != SMAUG_INT_EULER && B.stage > 0)) return;
+  const long c = (base ? tx : tx - 6) * nc + (long)gj * n0;
+  const int a = x0 < 2 ? 2 : x0, b = x0 + TX - 1 > n0 - 3 ? n0 - 3 : x0 + TX - 1;
+#pragma unroll
+  for (int k = 0; k < TX * 8 / 128 + 1; k++) {
+    const int x = a + 16 * k < b ? a + 16 * k : b;
+    const void* p = base ? static_cast<const void*>(static_cast<const ST*>(B.un) + c + x)
+                         : static_cast<const void*>(B.acc + c + x);
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
   }
 }
 
@@ -344,6 +333,8 @@ __device__ __forceinline__ bool stage2d_body(const KParams& P, const KBufs& B, i
   const bool inner = x0 - HALO >= 0 && by >= 1 && x0 - HALO + RX <= n0 && y0 + TY + HALO <= n1;
   // running CFL maxima of the grid when the block starts
   double seen[2];
+  __shared__ unsigned long long red[2];
+  __shared__ int arrived;
   {
     const unsigned long long* cm = B.cmax_out;
     seen[0] = __longlong_as_double(__ldcg(cm));
@@ -429,48 +420,60 @@ __device__ __forceinline__ bool stage2d_body(const KParams& P, const KBufs& B, i
     if (first) B.cmax_clear[0] = B.cmax_clear[1] = B.cmax_clear[2] = 0ull;
   }
   __syncthreads();
+  if (tid == 0) {
+    // after the barrier: every warp is done with the block's previous tile
+    red[0] = red[1] = 0ull;
+    arrived = 0;
+  }
   if constexpr (TMA) {
     if (tid == 0 && tt->nbx >= 0) tma_stage_issue<BG, MIX>(raw, rawb, *tt, tt->nbx, tt->nby);
   }
 
-  // ---- phase 1: centred fluxes -------------------------------------------
-  for (int u = tid; u < L::FXN + L::FYN; u += NTHREADS) {
-    const bool fx = u < L::FXN;
-    const int v = fx ? u : u - L::FXN;
-    const int lx = fx ? HALO - L::FH + v % L::FXW : HALO + v % TX;
-    const int ly = fx ? HALO + v / L::FXW : HALO - 2 + v / TX;
-    const int r = ly * QX + lx;
-    double g[4] = {0, 0, 0, 0}, f[5];
-    if (BG) {
-      const int gi = x0 - HALO + lx, gj = y0 - HALO + ly;
-      if (inner || (gi >= 0 && gi < n0 && gj >= 0 && gj < n1)) {
-        const long c = (long)gj * n0 + gi;
-        g[0] = __ldg(B.bg + c);
-        g[2] = __ldg(B.bg + 2 * nc + c);
-        g[3] = __ldg(B.bg + 3 * nc + c);
-      }
-    }
-    double* const o = fx ? F + v : F + 5 * L::FXN + v;
-    const int n = fx ? L::FXN : L::FYN;
-    if (fx)
-      s2::flux_at<BG, MIX, O6, 0>(sm, P.gamma, r, g, f);
-    else
-      s2::flux_at<BG, MIX, O6, 1>(sm, P.gamma, r, g, f);
-#pragma unroll
-    for (int k = 0; k < 5; k++) o[k * n] = f[k];
-  }
-  __syncthreads();
-
-  // ---- phase 2: divergence at the own cell --------------------------------
   const int lxo = tx + HALO, lyo = ty + HALO, ro = lyo * QX + lxo;
   const int gi = x0 + tx, gj = y0 + ty;
   const bool active = (XORG >= 2 || gi >= 2) && gi <= n0 - 3 && gj <= n1 - 3;
   const long co = active ? (long)gj * n0 + gi : 0;
+  double gb[4] = {0, 0, 0, 0};  // background fields at the tile cell
+
+  // ---- phase 1: centred fluxes: both directions at the own cell, then the
+  // cells beside the tile, one direction each -------------------------------
+  auto back = [&](int lx, int ly, double* g) {
+    const int ci = x0 - HALO + lx, cj = y0 - HALO + ly;
+    if (inner || (ci >= 0 && ci < n0 && cj >= 0 && cj < n1)) {
+      const long c = (long)cj * n0 + ci;
+      g[0] = __ldg(B.bg + c);
+      g[2] = __ldg(B.bg + 2 * nc + c);
+      g[3] = __ldg(B.bg + 3 * nc + c);
+    }
+  };
+  if (BG) {
+    back(lxo, lyo, gb);
+    if (active) gb[1] = __ldg(B.bg + nc + co);
+  }
+  s2::flux_at<BG, MIX, O6, true, true>(sm, P.gamma, ro, gb, F + ty * L::FXW + tx + L::FH, L::FXN,
+                                       F + 5 * L::FXN + (ty + 2) * TX + tx, L::FYN);
+  constexpr int NHY = 4 * TX, NHX = 2 * L::FH * TY;
+  for (int u = tid; u < NHY + NHX; u += NTHREADS) {
+    double g[4] = {0, 0, 0, 0};
+    if (u < NHY) {
+      const int row = u / TX, fr = row < 2 ? row : row + TY, col = u % TX;  // flux row 0, 1, TY+2, TY+3
+      if (BG) back(HALO + col, HALO - 2 + fr, g);
+      s2::flux_at<BG, MIX, O6, false, true>(sm, P.gamma, (HALO - 2 + fr) * QX + HALO + col, g, nullptr, 0,
+                                            F + 5 * L::FXN + fr * TX + col, L::FYN);
+    } else {
+      const int v = u - NHY, c = v % (2 * L::FH), fc = c < L::FH ? c : c + TX, row = v / (2 * L::FH);
+      if (BG) back(HALO - L::FH + fc, HALO + row, g);
+      s2::flux_at<BG, MIX, O6, true, false>(sm, P.gamma, (HALO + row) * QX + HALO - L::FH + fc, g,
+                                            F + row * L::FXW + fc, L::FXN, nullptr, 0);
+    }
+  }
+  __syncthreads();
+
+  // ---- phase 2: divergence at the own cell --------------------------------
   const HT* const qo = reinterpret_cast<const HT*>(sm + L::Q) + ro;
   const double rd0 = RD0[lxo], rd1 = RD1[lyo];
   const bool z0 = (P.bt[0] != 0) && zero1n(gi, n0), z1 = (P.bt[1] != 0) && zero1n(gj, n1);
   double out[6];
-  double gb[4] = {0, 0, 0, 0};  // background fields at the tile cell
   {
     const double kx = ((P.bt[0] != 0) && zero3dn(gi, n0)) || (O6 && edge6(gi, n0)) ? 0.0
                                                                                   : dt * rd0 * (O6 ? 0.25 : 1.0 / 12.0);
@@ -478,7 +481,7 @@ __device__ __forceinline__ bool stage2d_body(const KParams& P, const KBufs& B, i
     // 12 h times the 4th-order derivative; 4 h times the 6th-order one
     auto dx = [&](auto a) -> double {
       const double u1 = (double)a(1) - (double)a(-1), u2 = (double)a(-2) - (double)a(2);
-      if constexpr (O6) return 3.0 * u1 + 0.6 * u2 - ((double)a(-3) - (double)a(3)) * (1.0 / 15.0);
+      if constexpr (O6) return fma(3.0, u1, fma(0.6, u2, mulr((double)a(3) - (double)a(-3), 1.0 / 15.0)));
       return fma(8.0, u1, u2);
     };
     auto dy = [&](auto a) -> double {
@@ -488,30 +491,29 @@ __device__ __forceinline__ bool stage2d_body(const KParams& P, const KBufs& B, i
     const double* const fy = F + 5 * L::FXN + (ty + 2) * TX + tx;
     auto ddx = [&](int k) { return dx([&](int s) { return fx[k * L::FXN + s]; }); };
     auto ddy = [&](int k) { return dy([&](int s) { return fy[k * L::FYN + s * TX]; }); };
-    out[RHO] = -(kx * ddx(0)) - ky * ddy(0);
-    out[M1] = -(kx * ddx(1)) - ky * ddy(1);
-    out[M2] = -(kx * ddx(2)) - ky * ddy(2);
-    out[EN] = -(kx * ddx(3)) - ky * ddy(3);
-    out[B2] = -(kx * ddx(4));
-    out[B1] = -(ky * ddy(4));
+    out[RHO] = fma(-ky, ddy(0), -mulr(kx, ddx(0)));
+    out[M1] = fma(-ky, ddy(1), -mulr(kx, ddx(1)));
+    out[M2] = fma(-ky, ddy(2), -mulr(kx, ddx(2)));
+    out[EN] = fma(-ky, ddy(3), -mulr(kx, ddx(3)));
+    out[B2] = -mulr(kx, ddx(4));
+    out[B1] = -mulr(ky, ddy(4));
     if (BG) {
-      if (active) {
-#pragma unroll
-        for (int f = 0; f < 4; f++) gb[f] = __ldg(B.bg + f * nc + co);
-      }
       // addenergyterms_cd2 (src/centdiff2.cu:80-115)
       auto vel = [&](int c, int s) -> double {
         if constexpr (MIX)
-          return (double)qo[(s2::QM1 + c) * QC + s] * reinterpret_cast<const double*>(sm + L::RI)[ro + s];
+          return mulr((double)qo[(s2::QM1 + c) * QC + s], reinterpret_cast<const double*>(sm + L::RI)[ro + s]);
         else
           return (double)qo[(s2::QV1 + c) * QC + s];
       };
-      const double v1x = kx * dx([&](int s) { return vel(0, s); }), v2x = kx * dx([&](int s) { return vel(1, s); });
-      const double v1y = ky * dy([&](int s) { return vel(0, s * QX); });
-      const double v2y = ky * dy([&](int s) { return vel(1, s * QX); });
-      const double ptb = (P.gamma - 1) * gb[0] - 0.5 * (P.gamma - 2) * (gb[2] * gb[2] + gb[3] * gb[3]);
-      out[EN] -= ptb * (v1x + v2y);
-      out[EN] += gb[2] * (gb[2] * v1x + gb[3] * v2x) + gb[3] * (gb[2] * v1y + gb[3] * v2y);
+      const double v1x = mulr(kx, dx([&](int s) { return vel(0, s); }));
+      const double v2x = mulr(kx, dx([&](int s) { return vel(1, s); }));
+      const double v1y = mulr(ky, dy([&](int s) { return vel(0, s * QX); }));
+      const double v2y = mulr(ky, dy([&](int s) { return vel(1, s * QX); }));
+      const double ptb =
+          fma(P.gamma - 1, gb[0], -mulr(0.5 * (P.gamma - 2), fma(gb[2], gb[2], mulr(gb[3], gb[3]))));
+      out[EN] = fma(-ptb, v1x + v2y, out[EN]);
+      out[EN] = fma(gb[2], fma(gb[2], v1x, mulr(gb[3], v2x)), out[EN]);
+      out[EN] = fma(gb[3], fma(gb[2], v1y, mulr(gb[3], v2y)), out[EN]);
     }
     if (P.has_grav) {
       // addgrav_cd2 (src/centdiff2.cu:118-154); m rho / rho_t = v rho
@@ -519,15 +521,15 @@ __device__ __forceinline__ bool stage2d_body(const KParams& P, const KBufs& B, i
       double v1, v2;
       if constexpr (MIX) {
         const double ri = reinterpret_cast<const double*>(sm + L::RI)[ro];
-        v1 = (double)qo[s2::QM1 * QC] * ri;
-        v2 = (double)qo[s2::QM2 * QC] * ri;
+        v1 = mulr((double)qo[s2::QM1 * QC], ri);
+        v2 = mulr((double)qo[s2::QM2 * QC], ri);
       } else {
         v1 = (double)qo[s2::QV1 * QC];
         v2 = (double)qo[s2::QV2 * QC];
       }
-      out[M1] += dt * P.g[0] * rho;
-      out[M2] += dt * P.g[1] * rho;
-      out[EN] += dt * (P.g[0] * v1 + P.g[1] * v2) * rho;
+      out[M1] = fma(dt * P.g[0], rho, out[M1]);
+      out[M2] = fma(dt * P.g[1], rho, out[M2]);
+      out[EN] = fma(dt * fma(P.g[0], v1, mulr(P.g[1], v2)), rho, out[EN]);
     }
   }
 
@@ -565,7 +567,7 @@ __device__ __forceinline__ bool stage2d_body(const KParams& P, const KBufs& B, i
         const int f0 = s * SL, n = TX + 1 - f0 < SL ? TX + 1 - f0 : SL;
         const HT* q = reinterpret_cast<const HT*>(sm + L::Q) + fld * QC + (row + HALO - 1) * QX + HALO - 1 + f0;
         HT* o = RR + k * L::RXN + row * L::RXW + f0;
-        s2::ratio_line<SL, 1, (TX + 1) % SL == 0>(q, n, [&](int i, HT r, HT dq) { o[i] = cr ? r : r * dq; });
+        ratio_line<SL, 1, (TX + 1) % SL == 0>(q, n, [&](int i, HT r, HT dq) { o[i] = cr ? r : r * dq; });
       } else {
         // columns of rho, e, v2 on the tile, of v1, b1 one more on each side
         const int v = u - NXT;
@@ -575,34 +577,41 @@ __device__ __forceinline__ bool stage2d_body(const KParams& P, const KBufs& B, i
         const int fld = k == 0 ? s2::QR : k == 1 ? s2::QE : k == 2 ? s2::QV2 : k == 3 ? s2::QV1 : s2::QB1;
         const HT* q = reinterpret_cast<const HT*>(sm + L::Q) + fld * QC + (HALO - 1) * QX + col + HALO - 1;
         HT* o = RR + 5 * L::RXN + k * L::RYN + col;
-        s2::ratio_line<TY + 1, QX, true>(q, TY + 1, [&](int i, HT r, HT dq) { o[i * L::RYW] = cr ? r : r * dq; });
+        ratio_line<TY + 1, QX, true>(q, TY + 1, [&](int i, HT r, HT dq) { o[i * L::RYW] = cr ? r : r * dq; });
       }
     }
     __syncthreads();
-    // ---- phase 4: cross arrays (zero outside [2, n-3] and next to the edges) -
+    // ---- phase 4: diffusive terms; cross arrays (zero outside [2, n-3] and
+    // next to the edges) of the own cell and of the cells beside the tile ------
     HT* const CX = RR + 5 * (L::RXN + L::RYN);
     HT* const CY = CX + L::NC * L::CXN;
-    for (int u = tid; u < L::CXN + L::CYN; u += NTHREADS) {
-      const bool xd = u < L::CXN;
-      const int v = xd ? u : u - L::CXN;
-      const int cx = xd ? v % TX + 1 : v % L::CYW, cy = xd ? v / TX : v / L::CYW + 1;  // tile cell + 1
+    const HT* const px = RR + (ty + 1) * L::RXW + tx + 1;
+    const HT* const py = RR + 5 * L::RXN + (ty + 1) * L::RYW + tx + 1;
+    s2::diffuse<BG, MIX, O6, 0>(sm, P.chyp, ro, z0 ? 0.0 : dt * cin[0] * rd0, px, L::RXN, 1, out);
+    s2::cross_at<BG, MIX, O6, 0>(sm, P.chyp, cin[0], z0 || !active, ro, px, L::RXN, 1, CX + (ty + 1) * TX + tx,
+                                 L::CXN);
+    s2::diffuse<BG, MIX, O6, 1>(sm, P.chyp, ro, z1 ? 0.0 : dt * cin[1] * rd1, py, L::RYN, L::RYW, out);
+    s2::cross_at<BG, MIX, O6, 1>(sm, P.chyp, cin[1], z1 || !active, ro, py, L::RYN, L::RYW,
+                                 CY + ty * L::CYW + tx + 1, L::CYN);
+    for (int u = tid; u < 2 * TX + 2 * TY; u += NTHREADS) {
+      const bool xd = u < 2 * TX;
+      // tile cell + 1: rows 0 and TY+1 of the x passes, columns 0 and TX+1 of the y passes
+      const int v = u - 2 * TX;
+      const int cx = xd ? u % TX + 1 : (v & 1) * (TX + 1), cy = xd ? u / TX * (TY + 1) : v / 2 + 1;
       const int ci = x0 - 1 + cx, cj = y0 - 1 + cy;
       const int r = (cy + HALO - 1) * QX + cx + HALO - 1;
       const bool out2 = ci < 2 || ci > n0 - 3 || cj < 2 || cj > n1 - 3;
       if (xd)
         s2::cross_at<BG, MIX, O6, 0>(sm, P.chyp, cin[0], out2 || ((P.bt[0] != 0) && zero1n(ci, n0)), r,
-                                     RR + cy * L::RXW + cx, L::RXN, 1, CX + v, L::CXN);
+                                     RR + cy * L::RXW + cx, L::RXN, 1, CX + cy * TX + cx - 1, L::CXN);
       else
         s2::cross_at<BG, MIX, O6, 1>(sm, P.chyp, cin[1], out2 || ((P.bt[1] != 0) && zero1n(cj, n1)), r,
-                                     RR + 5 * L::RXN + cy * L::RYW + cx, L::RYN, L::RYW, CY + v, L::CYN);
+                                     RR + 5 * L::RXN + cy * L::RYW + cx, L::RYN, L::RYW,
+                                     CY + (cy - 1) * L::CYW + cx, L::CYN);
     }
-    __syncthreads();
-    // ---- phase 5: diffusive and cross terms ----------------------------------
     load_base();
-    s2::diffuse<BG, MIX, O6, 0>(sm, P.chyp, ro, z0 ? 0.0 : dt * cin[0] * rd0, RR + (ty + 1) * L::RXW + tx + 1,
-                                L::RXN, 1, out);
-    s2::diffuse<BG, MIX, O6, 1>(sm, P.chyp, ro, z1 ? 0.0 : dt * cin[1] * rd1,
-                                RR + 5 * L::RXN + (ty + 1) * L::RYW + tx + 1, L::RYN, L::RYW, out);
+    __syncthreads();
+    // ---- phase 5: cross terms --------------------------------------------------
     {
       // d/dy of the x passes' arrays, d/dx of the y passes'
       const double ky = z1 ? 0.0 : 0.5 * dt * rd1, kx = z0 ? 0.0 : 0.5 * dt * rd0;
@@ -643,17 +652,17 @@ __device__ __forceinline__ bool stage2d_body(const KParams& P, const KBufs& B, i
         v *= exp(-x * x / (P.drv_sigma[1] * P.drv_sigma[1]));
       }
       const double rr = rk ? (double)qo[s2::QR * QC] : ub[RHO] + out[RHO];
-      out[M1] = out[M1] + dt * v * (rr + gb[1]);
+      out[M1] = fma(dt * v, rr + gb[1], out[M1]);
     }
 #pragma unroll
     for (int f = 0; f < 6; f++) {
       if (!rk) {
         res[f] = ub[f] + out[f];
       } else if (B.stage == 3) {
-        res[f] = ac[f] + wgt * out[f];
+        res[f] = fma(wgt, out[f], ac[f]);
       } else {
-        B.acc[f * nc + co] = (B.stage == 0 ? ub[f] : ac[f]) + wgt * out[f];
-        res[f] = ub[f] + cst * out[f];
+        B.acc[f * nc + co] = fma(wgt, out[f], B.stage == 0 ? ub[f] : ac[f]);
+        res[f] = fma(cst, out[f], ub[f]);
       }
     }
     int hmax = 0;  // largest exponent word: infinities and NaN have 0x7ff
@@ -704,12 +713,24 @@ __device__ __forceinline__ bool stage2d_body(const KParams& P, const KBufs& B, i
         }
     }
   }
-  // maxima above what the grid had when the block started
+  // Maxima of the block, without a barrier: every warp adds its own to a shared
+  // pair, and the last one hands the pair on if it exceeds what the grid had
+  // when the block started.
   if (__any_sync(0xffffffffu, cm[0] > seen[0] || cm[1] > seen[1])) {
 #pragma unroll
     for (int d = 0; d < 2; d++) {
       for (int o = 16; o > 0; o >>= 1) cm[d] = dmax0(cm[d], __shfl_xor_sync(0xffffffffu, cm[d], o));
-      if ((tid & 31) == 0) atomicMax(&B.cmax_out[d], (unsigned long long)__double_as_longlong(cm[d]));
+      if ((tid & 31) == 0) atomicMax(&red[d], (unsigned long long)__double_as_longlong(cm[d]));
+    }
+  }
+  if ((tid & 31) == 0) {
+    __threadfence_block();
+    if (atomicAdd(&arrived, 1) == NTHREADS / 32 - 1) {
+#pragma unroll
+      for (int d = 0; d < 2; d++) {
+        const unsigned long long m = atomicMax(&red[d], 0ull);
+        if (__longlong_as_double(m) > seen[d]) atomicMax(&B.cmax_out[d], m);
+      }
     }
   }
   return true;
