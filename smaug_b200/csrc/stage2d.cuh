@@ -35,7 +35,13 @@
 //      have them
 //   5  own cell: cross terms, driver, stage sum, stores, ghost images, CFL
 //      maxima
-// The arrays of phases 1-2 and 3-5 share their memory.
+// The arrays of phases 1-2 and 3-5 share their memory (66 KB in FP64 without
+// background fields: three blocks of 256 threads at 80 registers).
+//
+// Bound by issue and latency, not by HBM: 57 warp instructions per cell and
+// stage at 49 % issue.  With every pass on its own the kernel took 109 at 60 %.
+// RK4 per step then and now: 4096^2 FP64 10.50 and 6.43 ms (2.3 ms at the
+// measured copy bandwidth), 64^2 0.092 and 0.049, 2048^2 mixed 2.46 and 1.40.
 #pragma once
 
 // (included inside namespace smaug)

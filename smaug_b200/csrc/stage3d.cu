@@ -1,5 +1,7 @@
 // stage3d.cu -- translation unit of the 3D stage kernel (stage3d.cuh)
 // and its launch dispatcher.
+#include <type_traits>
+
 #include "kernels.cuh"
 
 namespace smaug {

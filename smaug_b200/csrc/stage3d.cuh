@@ -1,7 +1,7 @@
 // stage3d.cuh -- fused 3D stage kernel, included by stage3d.cu.
 //
 // One launch evaluates the reference's whole spatial operator (the 3D build,
-// -DUSE_SAC_3D, of src/iosmaug.c:631-835) for an 8x8x4 tile of interior
+// -DUSE_SAC_3D, of src/iosmaug.c:631-835) for an 8x8x8 tile of interior
 // cells and writes the stage result, its ghost images and the per-dimension
 // fast-speed maxima.  The terms and their arithmetic are those of the 2D
 // kernel (stage2d.cuh) with three momentum and field components:
@@ -20,15 +20,23 @@
 // form (template MIX) is the one of stage2d.cuh: float perturbation storage
 // and hyperdiffusion arithmetic, double everywhere else.
 //
-// The state is read from global memory (L1/L2 resident across the passes of
-// a block); shared memory holds 1/rho_t and q on the tile's 3-cell box,
-// the per-axis metric, and one union of phase scratch:
+// The state is read from global memory (L1/L2 resident across the phases of
+// a block).  Shared memory holds 1/rho_t on the tile's 3-cell box, rho_t on the
+// tile +-1, the per-axis metric, the box cells' sources, and one union of phase
+// scratch:
 //   flux phase:  7 flux arrays + 3 velocity arrays on the tile +-2 along the
 //                direction
-//   hyperdiffusion phase: q of one field on the box (shared by the passes
-//                of all directions), the nu ratio on the tile +-1 across the
-//                direction extended by one cell along it, two cross-term
-//                arrays on the tile +-1 across the direction.
+//   hyperdiffusion, field by field: q on the box, the nu ratios of the field's
+//                passes (tile +-1 along the field's component only, which is
+//                where its cross terms are differentiated), three cross arrays
+// Bound by loads of the state from L2 and the barriers between the phases: 235
+// warp instructions per cell and stage at 35 % issue (494 at 48 % with 8x8x4
+// tiles and every pass on its own).  RK4 per step at 256^3 then and now: FP64
+// 61.1 and 37.5 ms, mixed 54 and 38.  Other tiles now: 16x8x4 40.5, 8x8x4 45.8.
+//
+// A field takes three block barriers: q staged | ratios of all directions, one
+// thread per piece of a line (ratio_line) | diffusive terms and cross arrays |
+// cross terms beside the staging of the next field.
 #pragma once
 
 // (included inside namespace smaug)
@@ -40,17 +48,23 @@ namespace s3 {
 #define SMAUG_T3Y 8
 #endif
 #ifndef SMAUG_T3Z
-#define SMAUG_T3Z 4
+#define SMAUG_T3Z 8
 #endif
 #ifndef SMAUG_MINB3D
-#define SMAUG_MINB3D 3  // resident blocks per SM the 3D stage is compiled for
+#define SMAUG_MINB3D 2  // resident blocks per SM the 3D stage is compiled for
+#endif
+#ifndef SMAUG_NB3
+#define SMAUG_NB3 3  // box cells of a thread whose loads are issued together
 #endif
 constexpr int T0 = SMAUG_T3X, T1 = SMAUG_T3Y, T2 = SMAUG_T3Z;  // tile (x fastest)
 constexpr int NT = T0 * T1 * T2;       // threads per block, one cell each
 constexpr int H = 3;                   // box halo
 constexpr int BX = T0 + 2 * H, BY = T1 + 2 * H, BZ = T2 + 2 * H;
-constexpr int BC = BX * BY * BZ;
-constexpr int BS1 = BX, BS2 = BX * BY;  // box strides
+// row pitch of the box arrays: odd, so that lines along x taken by
+// neighbouring threads fall on different banks
+constexpr int BP = BX | 1;
+constexpr int BC = BP * BY * BZ;
+constexpr int BS1 = BP, BS2 = BP * BY;  // box strides
 __host__ __device__ constexpr int max3(int a, int b, int c) {
   return a > b ? (a > c ? a : c) : (b > c ? b : c);
 }
@@ -59,21 +73,30 @@ template <bool O6>
 __host__ __device__ constexpr int fa() {
   return max3((T0 + (O6 ? 6 : 4)) * T1 * T2, T0 * (T1 + (O6 ? 6 : 4)) * T2, T0 * T1 * (T2 + (O6 ? 6 : 4)));
 }
-constexpr int NA = max3(T0 * (T1 + 2) * (T2 + 2), (T0 + 2) * T1 * (T2 + 2), (T0 + 2) * (T1 + 2) * T2);
-// ratio area: the nu area extended by one cell below along the direction
-constexpr int RA = max3((T0 + 1) * (T1 + 2) * (T2 + 2), (T0 + 2) * (T1 + 1) * (T2 + 2),
-                        (T0 + 2) * (T1 + 2) * (T2 + 1));
-constexpr int HYP_SCR = BC + RA + 2 * NA;
-constexpr int NMET = 2 * (BX + BY + BZ);
+// tile +-1 (rho_t), strides
+constexpr int EX = T0 + 2, EY = T1 + 2, EZ = T2 + 2, EC = EX * EY * EZ;
+// ratio areas: faces -1 .. T-1 along the direction, the tile across, one cell
+// more on each side along the field's component; cross arrays: the tile +-1
+// along the component
+constexpr int RA = max3((T0 + 1) * (T1 + 2) * T2, (T0 + 1) * T1 * (T2 + 2),
+                        max3((T0 + 2) * (T1 + 1) * T2, T0 * (T1 + 1) * (T2 + 2),
+                             max3((T0 + 2) * T1 * (T2 + 1), T0 * (T1 + 2) * (T2 + 1), 0)));
+constexpr int CA = max3((T0 + 2) * T1 * T2, T0 * (T1 + 2) * T2, T0 * T1 * (T2 + 2));
+constexpr int NMET = BX + BY + BZ;
+// cross arrays of one field: the two passes' momentum (or B) arrays and the
+// energy's, summed over the passes in double (the mixed form keeps both float
+// parts)
+template <bool MIX>
+__host__ __device__ constexpr int nca() { return MIX ? 4 : 3; }
 template <bool MIX, bool O6 = false>
 __host__ __device__ constexpr size_t union_bytes() {
-  return 10 * fa<O6>() * sizeof(double) > HYP_SCR * sizeof(typename Form<MIX>::H)
-             ? 10 * fa<O6>() * sizeof(double)
-             : HYP_SCR * sizeof(typename Form<MIX>::H);
+  constexpr size_t h = ((MIX ? 2 : 1) * BC + 3 * RA + nca<MIX>() * CA) * sizeof(typename Form<MIX>::H);
+  constexpr size_t f = 10 * fa<O6>() * sizeof(double);
+  return ((f > h ? f : h) + 7) / 8 * 8;
 }
 template <bool MIX, bool O6 = false>
 __host__ __device__ constexpr size_t smem_bytes() {
-  return sizeof(double) * (BC + NMET) + union_bytes<MIX, O6>() + sizeof(int) * BC;
+  return sizeof(double) * (BC + EC + NMET) + union_bytes<MIX, O6>() + sizeof(int) * BC;
 }
 __host__ __device__ constexpr int tdim(int d) { return d == 0 ? T0 : (d == 1 ? T1 : T2); }
 __host__ __device__ constexpr int bstride(int d) { return d == 0 ? 1 : (d == 1 ? BS1 : BS2); }
@@ -81,13 +104,17 @@ __host__ __device__ constexpr int bstride(int d) { return d == 0 ? 1 : (d == 1 ?
 
 struct Box3 {
   double* R;       // [BC] 1/rho_t on the box
-  double* dl[3];   // cell widths over the box extent of each axis
-  double* rd[3];   // reciprocals
+  double* T;       // [EC] rho_t on the tile +-1
+  double* rd[3];   // 1/dl over the box extent of each axis
   void* U;         // union scratch
   int* C;          // [BC] q source code per box cell (box_code)
   int o[3];        // global coordinate of box index 0 per axis
   bool inner;      // the box lies inside the grid and off its pads
 };
+// index into Box3::T of box cell (lx, ly, lz)
+__device__ __forceinline__ int eidx(int lx, int ly, int lz) {
+  return ((lz - s3::H + 1) * s3::EY + (ly - s3::H + 1)) * s3::EX + (lx - s3::H + 1);
+}
 
 // q of a hyperdiffusion field from global memory (src/hyperdifvisc1r.cu:1225-1253)
 template <typename ST, int KIND, int COMP>
@@ -95,7 +122,7 @@ __device__ __forceinline__ double hq3_global(const ST* u, const KBufs& B, long n
   const double rho = __ldg(u + c);
   if (KIND == 0) return rho;
   if (KIND == 3) return __ldg(u + (B3 + COMP) * nc + c);
-  const double r = 1.0 / (rho + __ldg(B.bg + GRB * nc + c));
+  const double r = recip(rho + __ldg(B.bg + GRB * nc + c));
   if (KIND == 2) return (double)__ldg(u + (M3 + COMP) * nc + c) * r;
   double m2 = 0, b2 = 0;
 #pragma unroll
@@ -123,33 +150,44 @@ __device__ __forceinline__ void stage_q(const Box3& X, const KParams& P, const K
   const ST* u = static_cast<const ST*>(B.uin);
   HT* Q = static_cast<HT*>(X.U);
   const long nc = P.ncell;
-  for (int r = tid; r < s3::BC; r += s3::NT) {
-    const int code = X.C[r];
-    double q = 0.0;
-    if (code >= 0) {
-      const long c = code;
-      if (KIND == 0) {
-        q = __ldg(u + c);
-      } else if (KIND == 3) {
-        q = __ldg(u + (B3 + COMP) * nc + c);
-      } else if (KIND == 2) {
-        q = (double)__ldg(u + (M3 + COMP) * nc + c) * X.R[r];
-      } else {
+  // a thread's cells in groups whose loads are all issued before their use; six
+  // at once (a whole thread) spill at 64 registers: 47.1 against 37.5 ms per RK4
+  // step at 256^3
+  constexpr int NI = (s3::BC + s3::NT - 1) / s3::NT, NB = KIND == 1 ? 1 : SMAUG_NB3, NF = KIND == 1 ? 7 : 1;
+  constexpr int F0 = KIND == 0 ? R3 : KIND == 1 ? M3 : KIND == 2 ? M3 + COMP : B3 + COMP;
+#pragma unroll 1
+  for (int i0 = 0; i0 < NI; i0 += NB) {
+    int code[NB];
+    ST w[NB][NF];
+#pragma unroll
+    for (int i = 0; i < NB; i++) {
+      const int r = tid + (i0 + i) * s3::NT;
+      code[i] = r < s3::BC ? X.C[r] : -1;
+#pragma unroll
+      for (int f = 0; f < NF; f++) w[i][f] = code[i] >= 0 ? __ldg(u + (F0 + f) * nc + code[i]) : (ST)0;
+    }
+#pragma unroll
+    for (int i = 0; i < NB; i++) {
+      const int r = tid + (i0 + i) * s3::NT;
+      if (r >= s3::BC) continue;
+      double q = (double)w[i][0];
+      if (KIND == 2) q = mulr(q, X.R[r]);
+      if (KIND == 1) {
+        // m1 m2 m3 e b1 b2 b3
         double m2 = 0, b2 = 0;
 #pragma unroll
         for (int a = 0; a < 3; a++) {
-          const double m = __ldg(u + (M3 + a) * nc + c), b = __ldg(u + (B3 + a) * nc + c);
-          m2 += m * m;
-          b2 += b * b;
+          const double m = (double)w[i][a], b = (double)w[i][NF - 3 + a];
+          m2 = fma(m, m, m2);
+          b2 = fma(b, b, b2);
         }
-        q = (double)__ldg(u + E3 * nc + c) - 0.5 * (b2 + m2 * X.R[r]);
+        q = fma(-0.5, fma(m2, X.R[r], b2), (double)w[i][NF / 2]);
       }
-    } else if (code <= -2) {
-      q = hq3_global<ST, KIND, COMP>(u, B, nc, (long)(-2 - code));
+      if (code[i] <= -2) q = hq3_global<ST, KIND, COMP>(u, B, nc, (long)(-2 - code[i]));
+      Q[r] = (HT)q;
+      if (MIX && KIND == 2) Q[s3::BC + r] = (HT)w[i][0];
     }
-    Q[r] = (HT)q;
   }
-  __syncthreads();
 }
 
 // Source code of box cell r for the q stagings (computed once per block):
@@ -180,157 +218,206 @@ __device__ __forceinline__ int box_code(const Box3& X, const KParams& P, const K
   return src >= 0 ? -2 - src : -1;
 }
 
-// One hyperdiffusion pass on staged q: field kind (0 rho, 1 energy,
-// 2 momentum, 3 B), component COMP, direction DIM.
+// Geometry of the passes of field (KIND, COMP) along DIM.
+template <int KIND, int COMP, int DIM>
+struct Pass3 {
+  static constexpr bool CROSS = (KIND == 2 && COMP != DIM) || KIND == 3;
+  static constexpr bool ON = !(KIND == 3 && COMP == DIM);  // B is not diffused along itself
+  static constexpr int X0 = CROSS && COMP == 0, X1 = CROSS && COMP == 1, X2 = CROSS && COMP == 2;
+  // ratio area: extents and box coordinates of its first cell
+  static constexpr int E0 = s3::T0 + (DIM == 0) + 2 * X0, E1 = s3::T1 + (DIM == 1) + 2 * X1;
+  static constexpr int E2 = s3::T2 + (DIM == 2) + 2 * X2;
+  static constexpr int G0 = s3::H - (DIM == 0) - X0, G1 = s3::H - (DIM == 1) - X1, G2 = s3::H - (DIM == 2) - X2;
+  static constexpr int RS = DIM == 0 ? 1 : (DIM == 1 ? E0 : E0 * E1);  // stride along DIM
+  static constexpr int SD = s3::bstride(DIM);
+  // lines along DIM, cut into two pieces of SL faces (the last may be shorter)
+  static constexpr int N = s3::tdim(DIM) + 1, SL = (N + 1) / 2;
+  static constexpr int A1 = DIM == 0 ? E1 : E0, A2 = DIM == 2 ? E1 : E2, NL = ON ? A1 * A2 * 2 : 0;
+  __device__ __forceinline__ static int ridx(int lx, int ly, int lz) {
+    return ((lz - G2) * E1 + (ly - G1)) * E0 + (lx - G0);
+  }
+};
+// cross arrays of component COMP: the tile +-1 along it
+template <int COMP>
+__device__ __forceinline__ int cidx3(int lx, int ly, int lz) {
+  constexpr int X0 = COMP == 0, X1 = COMP == 1, X2 = COMP == 2;
+  return ((lz - s3::H + X2) * (s3::T1 + 2 * X1) + (ly - s3::H + X1)) * (s3::T0 + 2 * X0) + (lx - s3::H + X0);
+}
+
+// piece u of the ratio lines of one pass: R where the pass has cross terms,
+// R (q(l+1) - q(l)) where it has none
 template <bool MIX, int KIND, int COMP, int DIM>
-__device__ __forceinline__ void hyper_pass3(const Box3& X, const KParams& P, const KBufs& B, int tid,
-                                            bool active, const int* lt, const int* gt, double dt,
-                                            double* out) {
-  constexpr bool CROSS = (KIND == 2 && COMP != DIM) || (KIND == 3);
-  constexpr int QFIELD = (KIND == 0) ? R3 : (KIND == 1) ? E3 : (KIND == 2) ? M3 + COMP : B3 + COMP;
-  constexpr int SD = s3::bstride(DIM);
-  // nu area: the tile along DIM, +-1 across when cross terms need it
-  constexpr int E0 = s3::T0 + ((CROSS && DIM != 0) ? 2 : 0);
-  constexpr int E1 = s3::T1 + ((CROSS && DIM != 1) ? 2 : 0);
-  constexpr int E2 = s3::T2 + ((CROSS && DIM != 2) ? 2 : 0);
-  constexpr int G0 = s3::H - ((CROSS && DIM != 0) ? 1 : 0);
-  constexpr int G1 = s3::H - ((CROSS && DIM != 1) ? 1 : 0);
-  constexpr int G2 = s3::H - ((CROSS && DIM != 2) ? 1 : 0);
-  constexpr int NAREA = E0 * E1 * E2;
-  // ratio area: the nu area extended by one cell below along DIM
-  constexpr int RE0 = E0 + (DIM == 0), RE1 = E1 + (DIM == 1), RE2 = E2 + (DIM == 2);
-  constexpr int RG0 = G0 - (DIM == 0), RG1 = G1 - (DIM == 1), RG2 = G2 - (DIM == 2);
-  constexpr int RAREA = RE0 * RE1 * RE2;
-  constexpr int RS = DIM == 0 ? 1 : (DIM == 1 ? RE0 : RE0 * RE1);  // stride along DIM in R
+__device__ __forceinline__ void ratio_piece(const Box3& X, int u) {
   using HT = typename Form<MIX>::H;
+  using G = Pass3<KIND, COMP, DIM>;
+  const int a = u % G::A1, v = u / G::A1, b = v % G::A2, f0 = v / G::A2 * G::SL;
+  int e[3];  // first face of the piece in the ratio area
+  e[DIM] = f0;
+  e[DIM == 0 ? 1 : 0] = a;
+  e[DIM == 2 ? 1 : 2] = b;
+  const int n = G::N - f0 < G::SL ? G::N - f0 : G::SL;
+  const HT* q = static_cast<const HT*>(X.U) + ((G::G2 + e[2]) * s3::BY + G::G1 + e[1]) * s3::BP + G::G0 + e[0];
+  HT* o = static_cast<HT*>(X.U) + (MIX ? 2 : 1) * s3::BC + DIM * s3::RA + (e[2] * G::E1 + e[1]) * G::E0 + e[0];
+  ratio_line<G::SL, G::SD, G::N % G::SL == 0>(q, n,
+                                              [&](int i, HT r, HT dq) { o[i * G::RS] = G::CROSS ? r : mulr(r, dq); });
+}
+template <bool MIX, int KIND, int COMP>
+__device__ __forceinline__ void ratios3(const Box3& X, int tid) {
+  constexpr int N0 = Pass3<KIND, COMP, 0>::NL, N1 = Pass3<KIND, COMP, 1>::NL, N2 = Pass3<KIND, COMP, 2>::NL;
+  // each direction's pieces start at a warp of their own where that takes no
+  // more rounds of the block
+  constexpr int P0 = (N0 + 31) / 32 * 32, P1 = P0 + (N1 + 31) / 32 * 32;
+  for (int u = tid; u < P1 + N2; u += s3::NT) {
+    if (u < P0) {
+      if (N0 > 0 && u < N0) ratio_piece<MIX, KIND, COMP, 0>(X, u);
+    } else if (u < P1) {
+      if (N1 > 0 && u - P0 < N1) ratio_piece<MIX, KIND, COMP, 1>(X, u - P0);
+    } else {
+      if (N2 > 0) ratio_piece<MIX, KIND, COMP, 2>(X, u - P1);
+    }
+  }
+}
+
+// Diffusive terms of one pass at the tile cell (hyperdif*source1):
+// dt cmax/dl (G(i) - G(i-1)), G = chyp R dq times the face mean
+template <bool BG, bool MIX, int KIND, int COMP, int DIM>
+__device__ __forceinline__ void diffuse3(const Box3& X, const KParams& P, const int* lt, double k, double* out) {
+  using HT = typename Form<MIX>::H;
+  using G = Pass3<KIND, COMP, DIM>;
+  if constexpr (G::ON) {
+    constexpr int S = G::SD;
+    const HT* q = static_cast<const HT*>(X.U) + (lt[2] * s3::BY + lt[1]) * s3::BP + lt[0];
+    const HT* r = static_cast<const HT*>(X.U) + (MIX ? 2 : 1) * s3::BC + DIM * s3::RA + G::ridx(lt[0], lt[1], lt[2]);
+    HT fp = r[0], fm = r[-G::RS];
+    if constexpr (G::CROSS) {
+      fp = mulr(fp, q[S] - q[0]);
+      fm = mulr(fm, q[0] - q[-S]);
+    }
+    if constexpr (KIND == 0) {
+      out[R3] = fma(k * P.chyp[R3], (double)(fp - fm), out[R3]);
+    } else if constexpr (KIND == 1) {
+      out[E3] = fma(k * P.chyp[E3], (double)(fp - fm), out[E3]);
+    } else if constexpr (KIND == 2) {
+      // the pass along the own component counts twice; face means carry 1/2
+      constexpr int ES = DIM == 0 ? 1 : (DIM == 1 ? s3::EX : s3::EX * s3::EY);
+      const double* t = X.T + eidx(lt[0], lt[1], lt[2]);
+      HT rp, rm, mp, mm;
+      if constexpr (MIX) {
+        rp = (HT)(t[0] + t[ES]);
+        rm = (HT)(t[-ES] + t[0]);
+        mp = q[s3::BC] + q[s3::BC + S];
+        mm = q[s3::BC - S] + q[s3::BC];
+      } else {
+        rp = t[0] + t[ES];
+        rm = t[-ES] + t[0];
+        const HT m0 = mulr(q[0], t[0]);
+        mp = fma(q[S], t[ES], m0);
+        mm = fma(q[-S], t[-ES], m0);
+      }
+      const double kk = (COMP == DIM ? 0.5 : 0.25) * k * P.chyp[M3 + COMP];
+      out[M3 + COMP] = fma(kk, (double)fma(fp, rp, -mulr(fm, rm)), out[M3 + COMP]);
+      out[E3] = fma(kk, (double)fma(fp, mp, -mulr(fm, mm)), out[E3]);
+    } else {
+      const double kk = k * P.chyp[B3 + COMP];
+      out[B3 + COMP] = fma(kk, (double)(fp - fm), out[B3 + COMP]);
+      out[E3] = fma(0.5 * kk, (double)fma(fp, q[0] + q[S], -mulr(fm, q[-S] + q[0])), out[E3]);
+    }
+  }
+}
+
+// Cross arrays of field (KIND, COMP) at one box cell (hyperdifmomsourcene2-4,
+// hyperdifbsourcene1b-4): for the passes along the two other dimensions a,
+// momentum: rho_t tau_a, and tau_a m_a for the energy; B: t_a, and t_a b_a, with
+// tau = (q+ - q-) (R + R-) cmax chyp / 8, t: / 4.  Zero outside [2, n-3] and, per
+// pass, next to a non-periodic edge along it.
+// ma: m or b of the two passes' dimensions at the cell.
+template <bool MIX, int KIND, int COMP>
+__device__ __forceinline__ void cross3(const Box3& X, const KParams& P, const KBufs& B, const int* l,
+                                       const typename Form<MIX>::S* ma) {
+  using HT = typename Form<MIX>::H;
+  const int n[3] = {P.n0, P.n1, P.n2};
+  const int g[3] = {X.o[0] + l[0], X.o[1] + l[1], X.o[2] + l[2]};
+  const bool in = g[0] >= 2 && g[0] <= n[0] - 3 && g[1] >= 2 && g[1] <= n[1] - 3 && g[2] >= 2 && g[2] <= n[2] - 3;
+  const HT* q = static_cast<const HT*>(X.U) + (l[2] * s3::BY + l[1]) * s3::BP + l[0];
+  HT* c = static_cast<HT*>(X.U) + (MIX ? 2 : 1) * s3::BC + 3 * s3::RA + cidx3<COMP>(l[0], l[1], l[2]);
+  HT v[4] = {0, 0, 0, 0};
+  if (in) {
+    constexpr int DA = COMP == 0 ? 1 : 0, DB = COMP == 2 ? 1 : 2;
+    auto pass = [&](auto dim, HT m, HT& f, HT& e) {
+      constexpr int D = decltype(dim)::value;
+      using G = Pass3<KIND, COMP, D>;
+      if ((P.bt[D] != 0) && zero1n(g[D], n[D])) return;
+      const HT* r = static_cast<const HT*>(X.U) + (MIX ? 2 : 1) * s3::BC + D * s3::RA + G::ridx(l[0], l[1], l[2]);
+      const HT k = (HT)((KIND == 2 ? 0.125 : 0.25) * B.cmax_in[D] * P.chyp[(KIND == 2 ? M3 : B3) + COMP]);
+      const HT t = (q[G::SD] - q[-G::SD]) * (r[0] + r[-G::RS]) * k;
+      f = KIND == 2 ? (HT)X.T[eidx(l[0], l[1], l[2])] * t : t;
+      e = mulr(t, m);
+    };
+    pass(std::integral_constant<int, DA>{}, (HT)ma[0], v[0], v[2]);
+    pass(std::integral_constant<int, DB>{}, (HT)ma[1], v[1], v[3]);
+  }
+  c[0] = v[0];
+  c[s3::CA] = v[1];
+  if constexpr (MIX) {
+    c[2 * s3::CA] = v[2];
+    c[3 * s3::CA] = v[3];
+  } else {
+    c[2 * s3::CA] = v[2] + v[3];
+  }
+}
+// the cross terms at the tile cell: d/dx_COMP of the arrays (sign - for B)
+template <bool MIX, int KIND, int COMP>
+__device__ __forceinline__ void cross_terms3(const Box3& X, const int* lt, double k, double* out) {
+  using HT = typename Form<MIX>::H;
+  constexpr int DA = COMP == 0 ? 1 : 0, DB = COMP == 2 ? 1 : 2, F = KIND == 2 ? M3 : B3;
+  constexpr int S = COMP == 0 ? 1 : (COMP == 1 ? s3::T0 : s3::T0 * s3::T1);
+  const HT* c = static_cast<const HT*>(X.U) + (MIX ? 2 : 1) * s3::BC + 3 * s3::RA + cidx3<COMP>(lt[0], lt[1], lt[2]);
+  auto d = [&](int i) -> double { return (double)(c[i * s3::CA + S] - c[i * s3::CA - S]); };
+  const double s = KIND == 2 ? k : -k;
+  out[F + DA] = fma(s, d(0), out[F + DA]);
+  out[F + DB] = fma(s, d(1), out[F + DB]);
+  out[E3] = fma(s, d(2), out[E3]);
+  if constexpr (MIX) out[E3] = fma(s, d(3), out[E3]);
+}
+
+// All passes of one field whose q has been staged (and not yet synchronised);
+// bit a of zero: the cell lies next to a non-periodic edge along a.  Leaves the cross terms to the caller (cross_terms3), so that they
+// run beside the next field's staging.
+template <bool BG, bool MIX, int KIND, int COMP>
+__device__ __forceinline__ void field3(const Box3& X, const KParams& P, const KBufs& B, int tid, const int* lt,
+                                       double dt, int zero, double* out) {
   using ST = typename Form<MIX>::S;
   const ST* u = static_cast<const ST*>(B.uin);
-  const int n[3] = {P.n0, P.n1, P.n2};
-  const long nc = P.ncell;
-  const HT* Q = static_cast<const HT*>(X.U);
-  HT* RR = static_cast<HT*>(X.U) + s3::BC;
-  HT* C3 = RR + s3::RA;
-  HT* C4 = C3 + s3::NA;
-  auto aidx = [&](int lx, int ly, int lz) { return ((lz - G2) * E1 + (ly - G1)) * E0 + (lx - G0); };
-  auto ridx = [&](int lx, int ly, int lz) { return ((lz - RG2) * RE1 + (ly - RG1)) * RE0 + (lx - RG0); };
-
-  // (B) nu_r(i) = c(i) R(i), nu_l(i) = c(i) R(i-1) with
-  // R(i) = max D3(i-1..i+1) / max D1(i-2..i+2) (hyperdifvisc2-4; the windows
-  // of nu_l(i) are those of nu_r(i-1)); 0 where the denominator is 0
-  const HT coef = (HT)(B.cmax_in[DIM] * P.chyp[QFIELD]);
-  for (int r = tid; r < RAREA; r += s3::NT) {
-    const int lx = RG0 + r % RE0, ly = RG1 + (r / RE0) % RE1, lz = RG2 + r / (RE0 * RE1);
-    const int q0 = (lz * s3::BY + ly) * s3::BX + lx;
-    HT q[6];
-#pragma unroll
-    for (int s = 0; s < 6; s++) q[s] = Q[q0 + (s - 2) * SD];
-    HT t4 = 0, t5 = 0;
-#pragma unroll
-    for (int k = 0; k < 3; k++)
-      t4 = hmax0(t4, (HT)fabs((HT)3 * (q[k + 2] - q[k + 1]) - (q[k + 3] - q[k])));
-#pragma unroll
-    for (int k = 0; k < 5; k++) t5 = hmax0(t5, (HT)fabs(q[k + 1] - q[k]));
-    RR[r] = (t5 > 0) ? hdiv(t4, t5) : (HT)0;
-  }
+  constexpr int F = KIND == 2 ? M3 : B3, DA = COMP == 0 ? 1 : 0, DB = COMP == 2 ? 1 : 2;
+  constexpr int T = s3::tdim(COMP), L = s3::NT / T;  // cells of a layer across the component
+  static_assert(2 * L <= s3::NT, "the two layers beside the tile take one round");
+  auto get = [&](const int* b, ST* m) {
+    const int g0 = X.o[0] + b[0], g1 = X.o[1] + b[1], g2 = X.o[2] + b[2];
+    if (g0 > P.n0 - 1 || g1 > P.n1 - 1 || g2 > P.n2 - 1) return;
+    const long c = ((long)g2 * P.n1 + g1) * P.n0 + g0;
+    m[0] = __ldg(u + (F + DA) * P.ncell + c);
+    m[1] = __ldg(u + (F + DB) * P.ncell + c);
+  };
   __syncthreads();
-  // (C) cross-term arrays (hyperdifmomsourcene2-4 / hyperdifbsourcene1b-4)
-  if (CROSS) {
-    for (int r = tid; r < NAREA; r += s3::NT) {
-      const int lx = G0 + r % E0, ly = G1 + (r / E0) % E1, lz = G2 + r / (E0 * E1);
-      const int g[3] = {X.o[0] + lx, X.o[1] + ly, X.o[2] + lz};
-      HT c3 = 0, c4 = 0;
-      if (X.inner ||
-          (g[0] > 0 && g[0] < n[0] - 1 && g[1] > 0 && g[1] < n[1] - 1 && g[2] > 0 && g[2] < n[2] - 1)) {
-        const int q0 = (lz * s3::BY + ly) * s3::BX + lx;
-        const int la = DIM == 0 ? lx : (DIM == 1 ? ly : lz);
-        // grad13n along DIM of q
-        HT gq = ((Q[q0 + SD] - Q[q0 - SD]) * (HT)X.rd[DIM][la]) * (HT)0.5;
-        if ((P.bt[DIM] != 0) && zero1n(g[DIM], n[DIM])) gq = 0;
-        HT nsum = 0;
-        if (X.inner || (g[0] >= 2 && g[0] <= n[0] - 3 && g[1] >= 2 && g[1] <= n[1] - 3 && g[2] >= 2 &&
-                        g[2] <= n[2] - 3)) {
-          const int rr = ridx(lx, ly, lz);
-          const HT cc = (HT)X.dl[DIM][la] * coef;
-          nsum = cc * RR[rr] + cc * RR[rr - RS];
-        }
-        const long c = ((long)g[2] * n[1] + g[1]) * n[0] + g[0];
-        if (KIND == 2) {
-          const HT tau = (gq * nsum) * (HT)0.25;
-          c3 = (HT)((double)__ldg(u + c) + __ldg(B.bg + GRB * nc + c)) * tau;
-          c4 = tau * (HT)__ldg(u + (M3 + DIM) * nc + c);
-        } else {
-          const HT t3 = (gq * nsum) * (HT)0.5;
-          c3 = t3;
-          c4 = t3 * (HT)__ldg(u + (B3 + DIM) * nc + c);
-        }
-      }
-      C3[r] = c3;
-      C4[r] = c4;
-    }
-    __syncthreads();
-  }
-  // (D) sources at the tile cells
-  if (active) {
-    const int la = lt[DIM];
-    const int q0 = (lt[2] * s3::BY + lt[1]) * s3::BX + lt[0];
-    const int nidx = aidx(lt[0], lt[1], lt[2]);
-    const int rr = ridx(lt[0], lt[1], lt[2]);
-    const HT cc = (HT)X.dl[DIM][la] * coef;
-    const HT nur = cc * RR[rr], nul = cc * RR[rr - RS];
-    const HT rdl = (HT)X.rd[DIM][la];
-    const HT qc = Q[q0], qp = Q[q0 + SD], qm = Q[q0 - SD];
-    HT gr = (qp - qc) * rdl;  // grad1r3n
-    HT gl = (qc - qm) * rdl;  // grad1l3n
-    if ((P.bt[DIM] != 0) && zero1n(gt[DIM], n[DIM])) { gr = 0; gl = 0; }
-    if (KIND == 0) {
-      out[R3] = out[R3] + dt * (double)((nur * gr - nul * gl) * rdl);
-    } else if (KIND == 1) {
-      out[E3] = out[E3] + dt * (double)((nur * gr - nul * gl) * rdl);
-    } else if (KIND == 2) {
-      // hyperdifmomsource1-3a (src/hyperdifmomsource1.cu:17-511), ii0 = COMP
-      const long c = ((long)gt[2] * n[1] + gt[1]) * n[0] + gt[0];
-      const long sd = DIM == 0 ? 1 : (DIM == 1 ? (long)n[0] : (long)n[0] * n[1]);
-      const ST* rho = u;
-      const double* rb = B.bg + GRB * nc;
-      const ST* mf = u + (M3 + COMP) * nc;
-      const double r0 = (double)__ldg(rho + c) + __ldg(rb + c);
-      const HT t2 = (HT)((r0 + (double)__ldg(rho + c - sd) + __ldg(rb + c - sd)) * 0.5);
-      const HT t3 = (HT)((r0 + (double)__ldg(rho + c + sd) + __ldg(rb + c + sd)) * 0.5);
-      const double m0 = __ldg(mf + c);
-      const HT t5 = (HT)((m0 + (double)__ldg(mf + c - sd)) * 0.5);
-      const HT t6 = (HT)((m0 + (double)__ldg(mf + c + sd)) * 0.5);
-      const double dm = (double)(((t3 * nur * gr - t2 * nul * gl) * rdl) * (HT)0.5);
-      const double de = (double)(((t6 * nur * gr - t5 * nul * gl) * rdl) * (HT)0.5);
-      out[M3 + COMP] = out[M3 + COMP] + dt * dm;
-      out[E3] = out[E3] + dt * de;
-      if (COMP == DIM) {
-        out[M3 + COMP] = out[M3 + COMP] + dt * dm;
-        out[E3] = out[E3] + dt * de;
-      } else {
-        // hyperdifmomsourcene5-6a: d/dx_COMP of (rho_t tau) and (tau m_DIM)
-        constexpr int FS = COMP == 0 ? 1 : (COMP == 1 ? E0 : E0 * E1);
-        const HT rdf = (HT)X.rd[COMP][lt[COMP]];
-        HT g7 = ((C3[nidx + FS] - C3[nidx - FS]) * rdf) * (HT)0.5;
-        HT g8 = ((C4[nidx + FS] - C4[nidx - FS]) * rdf) * (HT)0.5;
-        if ((P.bt[COMP] != 0) && zero1n(gt[COMP], n[COMP])) { g7 = 0; g8 = 0; }
-        out[M3 + DIM] = out[M3 + DIM] + dt * (double)g7;
-        out[E3] = out[E3] + dt * (double)g8;
-      }
-    } else {
-      // B component COMP diffused along DIM: hyperdifbsourcene (sb=-1) then
-      // hyperdifbsource (sb=+1)
-      constexpr int FS = COMP == 0 ? 1 : (COMP == 1 ? E0 : E0 * E1);
-      const HT rdf = (HT)X.rd[COMP][lt[COMP]];
-      HT g4 = ((C3[nidx + FS] - C3[nidx - FS]) * rdf) * (HT)0.5;
-      HT g6 = ((C4[nidx + FS] - C4[nidx - FS]) * rdf) * (HT)0.5;
-      if ((P.bt[COMP] != 0) && zero1n(gt[COMP], n[COMP])) { g4 = 0; g6 = 0; }
-      out[B3 + DIM] = out[B3 + DIM] - dt * (double)g4;
-      out[E3] = out[E3] - dt * (double)g6;
-      const HT t2 = (qc + qm) * (HT)0.5, t3 = (qc + qp) * (HT)0.5;
-      const double dB = (double)((gr * nur - gl * nul) * rdl);
-      const double de = (double)((t3 * gr * nur - t2 * gl * nul) * rdl);
-      out[B3 + COMP] = out[B3 + COMP] + dt * dB;
-      out[E3] = out[E3] + dt * de;
+  ratios3<MIX, KIND, COMP>(X, tid);
+  __syncthreads();
+  diffuse3<BG, MIX, KIND, COMP, 0>(X, P, lt, (zero >> 0) & 1 ? 0.0 : dt * B.cmax_in[0] * X.rd[0][lt[0]], out);
+  diffuse3<BG, MIX, KIND, COMP, 1>(X, P, lt, (zero >> 1) & 1 ? 0.0 : dt * B.cmax_in[1] * X.rd[1][lt[1]], out);
+  diffuse3<BG, MIX, KIND, COMP, 2>(X, P, lt, (zero >> 2) & 1 ? 0.0 : dt * B.cmax_in[2] * X.rd[2][lt[2]], out);
+  if constexpr (KIND >= 2) {
+    ST m[2] = {0, 0};
+    get(lt, m);
+    cross3<MIX, KIND, COMP>(X, P, B, lt, m);
+    if (tid < 2 * L) {
+      // the two layers beside the tile along the component
+      const int v = tid % L;
+      constexpr int A = COMP == 0 ? 1 : 0, C = COMP == 2 ? 1 : 2;
+      int l[3];
+      l[COMP] = s3::H + (tid < L ? -1 : T);
+      l[A] = s3::H + v % s3::tdim(A);
+      l[C] = s3::H + v / s3::tdim(A);
+      get(l, m);
+      cross3<MIX, KIND, COMP>(X, P, B, l, m);
     }
   }
   __syncthreads();
@@ -370,7 +457,7 @@ __device__ __forceinline__ void flux3(const double* s, const double* g, double r
 template <bool BG, bool MIX, int D, bool O6>
 __device__ __forceinline__ void flux_pass3(const Box3& X, const KParams& P, const KBufs& B, int tid,
                                            bool active, const int* lt, const int* gt, double dt,
-                                           const double* gc, double* out) {
+                                           double* out) {
   constexpr int FH = O6 ? 3 : 2, FA = s3::fa<O6>();
   constexpr int E0 = s3::T0 + (D == 0 ? 2 * FH : 0), E1 = s3::T1 + (D == 1 ? 2 * FH : 0);
   constexpr int E2 = s3::T2 + (D == 2 ? 2 * FH : 0);
@@ -395,7 +482,7 @@ __device__ __forceinline__ void flux_pass3(const Box3& X, const KParams& P, cons
 #pragma unroll
         for (int k = 0; k < 5; k++) g[k] = __ldg(B.bg + k * nc + c);
       }
-      flux3<BG, D>(s, g, X.R[(lz * s3::BY + ly) * s3::BX + lx], P.gamma, f, v);
+      flux3<BG, D>(s, g, X.R[(lz * s3::BY + ly) * s3::BP + lx], P.gamma, f, v);
     }
 #pragma unroll
     for (int k = 0; k < 7; k++) F[k * FA + r] = f[k];
@@ -405,10 +492,10 @@ __device__ __forceinline__ void flux_pass3(const Box3& X, const KParams& P, cons
     }
   }
   __syncthreads();
+  const bool z = ((P.bt[D] != 0) && zero3dn(gt[D], n[D])) || (O6 && edge6(gt[D], n[D]));
+  const double rdl2 = 0.5 * X.rd[D][lt[D]];
+  const int fo = ((lt[2] - G2) * E1 + (lt[1] - G1)) * E0 + (lt[0] - G0);
   if (active) {
-    const bool z = ((P.bt[D] != 0) && zero3dn(gt[D], n[D])) || (O6 && edge6(gt[D], n[D]));
-    const double rdl2 = 0.5 * X.rd[D][lt[D]];
-    const int fo = ((lt[2] - G2) * E1 + (lt[1] - G1)) * E0 + (lt[0] - G0);
     constexpr int c1 = D == 0 ? 1 : 0, c2 = D == 2 ? 1 : 2;
     const int fld[7] = {R3, M3, M3 + 1, M3 + 2, E3, B3 + c1, B3 + c2};
 #pragma unroll
@@ -420,8 +507,10 @@ __device__ __forceinline__ void flux_pass3(const Box3& X, const KParams& P, cons
     if (BG) {
       // addenergyterms_cd2 (src/centdiff2.cu:80-115): -p_tb dv_D/dx_D, and
       // the derivative-along-D part of sum_i Bb_i Bb_d dv_d/dx_i
-      const double bb[3] = {gc[2], gc[3], gc[4]};
-      const double ptb = (P.gamma - 1) * gc[0] - 0.5 * (P.gamma - 2) * (bb[0] * bb[0] + bb[1] * bb[1] + bb[2] * bb[2]);
+      const long co = ((long)gt[2] * n[1] + gt[1]) * n[0] + gt[0];
+      const double eb = __ldg(B.bg + GEB * nc + co);
+      const double bb[3] = {__ldg(B.bg + 2 * nc + co), __ldg(B.bg + 3 * nc + co), __ldg(B.bg + 4 * nc + co)};
+      const double ptb = (P.gamma - 1) * eb - 0.5 * (P.gamma - 2) * (bb[0] * bb[0] + bb[1] * bb[1] + bb[2] * bb[2]);
       double gv = dflux<O6>(F + (7 + D) * FA, fo, FS, rdl2);
       if (z) gv = 0;
       out[E3] -= dt * ptb * gv;
@@ -443,10 +532,8 @@ __global__ void __launch_bounds__(s3::NT, SMAUG_MINB3D) stage3d_fast(const KPara
   extern __shared__ double smem[];
   Box3 X;
   X.R = smem;
-  X.dl[0] = smem + s3::BC;
-  X.dl[1] = X.dl[0] + s3::BX;
-  X.dl[2] = X.dl[1] + s3::BY;
-  X.rd[0] = X.dl[2] + s3::BZ;
+  X.T = smem + s3::BC;
+  X.rd[0] = X.T + s3::EC;
   X.rd[1] = X.rd[0] + s3::BX;
   X.rd[2] = X.rd[1] + s3::BY;
   X.U = X.rd[2] + s3::BZ;
@@ -463,24 +550,62 @@ __global__ void __launch_bounds__(s3::NT, SMAUG_MINB3D) stage3d_fast(const KPara
   X.inner = X.o[0] >= 0 && X.o[1] >= 0 && X.o[2] >= 0 && X.o[0] + s3::BX <= n[0] &&
             X.o[1] + s3::BY <= n[1] && X.o[2] + s3::BZ <= n[2];
 
+  // running CFL maxima of the grid when the block starts
+  double seen[3];
+#pragma unroll
+  for (int d = 0; d < 3; d++)
+    seen[d] = __longlong_as_double(__ldcg(static_cast<const unsigned long long*>(B.cmax_out) + d));
+
   // ---- 1/rho_t on the box and the per-axis metric ----------------------
-  for (int r = tid; r < s3::BC; r += s3::NT) {
-    const int lx = r % s3::BX, ly = (r / s3::BX) % s3::BY, lz = r / s3::BS2;
-    const int g0 = X.o[0] + lx, g1 = X.o[1] + ly, g2 = X.o[2] + lz;
-    double rinv = 1.0;
-    if (X.inner || (g0 >= 0 && g0 < n[0] && g1 >= 0 && g1 < n[1] && g2 >= 0 && g2 < n[2])) {
-      const long c = ((long)g2 * n[1] + g1) * n[0] + g0;
-      rinv = 1.0 / ((double)__ldg(u + c) + __ldg(B.bg + GRB * nc + c));
+  {
+    constexpr int NI = (s3::BC + s3::NT - 1) / s3::NT, NB = SMAUG_NB3;
+#pragma unroll 1
+    for (int i0 = 0; i0 < NI; i0 += NB) {
+      ST rho[NB];
+      double rhob[NB];
+#pragma unroll
+      for (int i = 0; i < NB; i++) {
+        const int r = tid + (i0 + i) * s3::NT;
+        const int lx = r % s3::BP, ly = (r / s3::BP) % s3::BY, lz = r / s3::BS2;
+        const int g0 = X.o[0] + lx, g1 = X.o[1] + ly, g2 = X.o[2] + lz;
+        const bool in = r < s3::BC && lx < s3::BX &&
+                        (X.inner || (g0 >= 0 && g0 < n[0] && g1 >= 0 && g1 < n[1] && g2 >= 0 && g2 < n[2]));
+        const long c = in ? ((long)g2 * n[1] + g1) * n[0] + g0 : 0;
+        rho[i] = in ? __ldg(u + c) : (ST)1;
+        rhob[i] = in ? __ldg(B.bg + GRB * nc + c) : 0.0;
+        if (r < s3::BC) X.C[r] = lx < s3::BX ? box_code(X, P, B, lx, ly, lz) : -1;
+      }
+#pragma unroll
+      for (int i = 0; i < NB; i++) {
+        const int r = tid + (i0 + i) * s3::NT;
+        if (r >= s3::BC) continue;
+        const int lx = r % s3::BP, ly = (r / s3::BP) % s3::BY, lz = r / s3::BS2;
+        const double rt = (double)rho[i] + rhob[i];
+        X.R[r] = recip(rt);
+        if (outside(lx, s3::T0) <= 1 && outside(ly, s3::T1) <= 1 && outside(lz, s3::T2) <= 1)
+          X.T[eidx(lx, ly, lz)] = rt;
+      }
     }
-    X.R[r] = rinv;
-    X.C[r] = box_code(X, P, B, lx, ly, lz);
+  }
+  // the stage sum's operands into L2, a block's lifetime ahead: one thread per
+  // row of the tile and array
+  for (int r = tid; r < 16 * s3::T1 * s3::T2; r += s3::NT) {
+    const int f = r % 16, v = r / 16;
+    const int g1 = X.o[1] + s3::H + v % s3::T1, g2 = X.o[2] + s3::H + v / s3::T1;
+    const bool base = f < 8;
+    if (g1 <= n[1] - 3 && g2 <= n[2] - 3 &&
+        (base ? (MODE == SMAUG_INT_EULER || B.stage < 3) : (MODE != SMAUG_INT_EULER && B.stage > 0))) {
+      const long c = (f & 7) * nc + ((long)g2 * n[1] + g1) * n[0] + X.o[0] + s3::H;
+      const void* q = base ? static_cast<const void*>(static_cast<const ST*>(B.un) + c)
+                           : static_cast<const void*>(B.acc + c);
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(q));
+    }
   }
   for (int r = tid; r < s3::BX + s3::BY + s3::BZ; r += s3::NT) {
     const int a = r < s3::BX ? 0 : (r < s3::BX + s3::BY ? 1 : 2);
     const int l = r - (a == 0 ? 0 : (a == 1 ? s3::BX : s3::BX + s3::BY));
     const int g = X.o[a] + l;
     const double d = (g >= 0 && g < n[a]) ? B.delx[a][g] : 1.0;
-    X.dl[a][l] = d;
     X.rd[a][l] = 1.0 / d;
   }
 
@@ -507,61 +632,52 @@ __global__ void __launch_bounds__(s3::NT, SMAUG_MINB3D) stage3d_fast(const KPara
   const bool active = gt[0] <= n[0] - 3 && gt[1] <= n[1] - 3 && gt[2] <= n[2] - 3;
   const long co = active ? ((long)gt[2] * n[1] + gt[1]) * n[0] + gt[0] : 0;
 
-  double sc[8], gc[5] = {0, 0, 0, 0, 0};
+  double out[8];  // increments
 #pragma unroll
-  for (int f = 0; f < 8; f++) sc[f] = active ? (double)__ldg(u + f * nc + co) : 0.0;
-#pragma unroll
-  for (int f = 0; f < 5; f++) gc[f] = active ? __ldg(B.bg + f * nc + co) : 0.0;
-  double out[8];
-#pragma unroll
-  for (int f = 0; f < 8; f++) {
-    if (MODE != SMAUG_INT_EULER)
-      out[f] = 0.0;
-    else if (MIX)
-      out[f] = active ? base_value<MIX>(B, f * nc + co) : 0.0;
-    else
-      out[f] = sc[f];
-  }
+  for (int f = 0; f < 8; f++) out[f] = 0.0;
 
   // ---- fluxes and divergence, direction 0, 1, 2 ----------------------------
-  flux_pass3<BG, MIX, 0, O6>(X, P, B, tid, active, lt, gt, dt, gc, out);
-  flux_pass3<BG, MIX, 1, O6>(X, P, B, tid, active, lt, gt, dt, gc, out);
-  flux_pass3<BG, MIX, 2, O6>(X, P, B, tid, active, lt, gt, dt, gc, out);
+  flux_pass3<BG, MIX, 0, O6>(X, P, B, tid, active, lt, gt, dt, out);
+  flux_pass3<BG, MIX, 1, O6>(X, P, B, tid, active, lt, gt, dt, out);
+  flux_pass3<BG, MIX, 2, O6>(X, P, B, tid, active, lt, gt, dt, out);
 
   // ---- gravity (addgrav_cd2, src/centdiff2.cu:118-154) --------------------
   if (P.has_grav && active) {
-    const double rho = sc[R3];
-    out[M3 + 0] += dt * P.g[0] * rho;
-    out[M3 + 1] += dt * P.g[1] * rho;
-    out[M3 + 2] += dt * P.g[2] * rho;
-    const double rr = rho * X.R[(lt[2] * s3::BY + lt[1]) * s3::BX + lt[0]];
-    out[E3] += (dt * P.g[0] * sc[M3 + 0]) * rr;
-    out[E3] += (dt * P.g[1] * sc[M3 + 1]) * rr;
-    out[E3] += (dt * P.g[2] * sc[M3 + 2]) * rr;
+    const double rho = (double)__ldg(u + co);
+    const double rr = rho * X.R[(lt[2] * s3::BY + lt[1]) * s3::BP + lt[0]];
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      out[M3 + a] = fma(dt * P.g[a], rho, out[M3 + a]);
+      out[E3] = fma(dt * P.g[a] * (double)__ldg(u + (M3 + a) * nc + co), rr, out[E3]);
+    }
   }
 
-  // ---- hyperdiffusion: one q staging per field, then every direction ----
+  // ---- hyperdiffusion, field by field; a field's cross terms run beside the
+  // staging of the next --------------------------------------------------
   if (P.hyperdif == 1) {
-#define HP(K, C, D) hyper_pass3<MIX, K, C, D>(X, P, B, tid, active, lt, gt, dt, out)
-#define SQ(K, C) stage_q<MIX, K, C>(X, P, B, tid)
-    SQ(0, 0);
-    HP(0, 0, 0); HP(0, 0, 1); HP(0, 0, 2);
-    SQ(1, 0);
-    HP(1, 0, 0); HP(1, 0, 1); HP(1, 0, 2);
-    SQ(2, 0);
-    HP(2, 0, 0); HP(2, 0, 1); HP(2, 0, 2);
-    SQ(2, 1);
-    HP(2, 1, 0); HP(2, 1, 1); HP(2, 1, 2);
-    SQ(2, 2);
-    HP(2, 2, 0); HP(2, 2, 1); HP(2, 2, 2);
-    SQ(3, 0);
-    HP(3, 0, 1); HP(3, 0, 2);
-    SQ(3, 1);
-    HP(3, 1, 0); HP(3, 1, 2);
-    SQ(3, 2);
-    HP(3, 2, 0); HP(3, 2, 1);
-#undef SQ
-#undef HP
+    int zero = 0;  // directions next to whose non-periodic edge the cell lies
+#pragma unroll
+    for (int a = 0; a < 3; a++) zero |= ((P.bt[a] != 0) && zero1n(gt[a], n[a])) << a;
+#define FIELD(K, C)                      \
+  stage_q<MIX, K, C>(X, P, B, tid);      \
+  field3<BG, MIX, K, C>(X, P, B, tid, lt, dt, zero, out)
+#define CROSS(K, C) cross_terms3<MIX, K, C>(X, lt, (zero >> C) & 1 ? 0.0 : 0.5 * dt * X.rd[C][lt[C]], out)
+    FIELD(0, 0);
+    FIELD(1, 0);
+    FIELD(2, 0);
+    CROSS(2, 0);
+    FIELD(2, 1);
+    CROSS(2, 1);
+    FIELD(2, 2);
+    CROSS(2, 2);
+    FIELD(3, 0);
+    CROSS(3, 0);
+    FIELD(3, 1);
+    CROSS(3, 1);
+    FIELD(3, 2);
+    CROSS(3, 2);
+#undef FIELD
+#undef CROSS
   }
 
   // ---- user driver (source_parallel + addsourceterms2) ---------------------
@@ -575,40 +691,48 @@ __global__ void __launch_bounds__(s3::NT, SMAUG_MINB3D) stage3d_fast(const KPara
         v *= exp(-x * x / (P.drv_sigma[a] * P.drv_sigma[a]));
       }
     }
-    const double rr = (MODE == SMAUG_INT_EULER) ? out[R3] : sc[R3];
-    out[M3] = out[M3] + dt * v * (rr + gc[GRB]);
+    const double rr = (double)__ldg(u + co) + (MODE == SMAUG_INT_EULER ? out[R3] : 0.0);
+    out[M3] = fma(dt * v, rr + __ldg(B.bg + GRB * nc + co), out[M3]);
   }
 
   // ---- combine, write, ghost images, CFL maxima -----------------------------
-  double cm[3] = {P.cmax_floor[0], P.cmax_floor[1], P.cmax_floor[2]};
+  double cm[3];
+#pragma unroll
+  for (int d = 0; d < 3; d++) cm[d] = P.cmax_floor[d] > seen[d] ? P.cmax_floor[d] : seen[d];
   if (active) {
     double res[8];
     const bool is_base = (MODE == SMAUG_INT_EULER) || B.stage == 3;
+    // all loads before the first store (a load after a store to the
+    // accumulator would wait for its own round trip)
+    double ub[8], ac[8];
+    if (MODE == SMAUG_INT_EULER || B.stage < 3) {
+#pragma unroll
+      for (int f = 0; f < 8; f++) ub[f] = base_value<MIX>(B, f * nc + co);
+    }
+    if (MODE != SMAUG_INT_EULER && B.stage > 0) {
+#pragma unroll
+      for (int f = 0; f < 8; f++) ac[f] = B.acc[f * nc + co];
+    }
     if (MODE == SMAUG_INT_EULER) {
 #pragma unroll
-      for (int f = 0; f < 8; f++) res[f] = out[f];
+      for (int f = 0; f < 8; f++) res[f] = ub[f] + out[f];
     } else {
       const double wgt = (B.stage == 0 || B.stage == 3) ? 1.0 / 6.0 : 1.0 / 3.0;
       const double cst = (B.stage == 2) ? 1.0 : 0.5;
 #pragma unroll
       for (int f = 0; f < 8; f++) {
-        const double dl = out[f];
-        if (B.stage == 0) {
-          const double u0 = MIX ? base_value<MIX>(B, f * nc + co) : sc[f];
-          B.acc[f * nc + co] = u0 + wgt * dl;
-          res[f] = u0 + cst * dl;
-        } else if (B.stage < 3) {
-          B.acc[f * nc + co] = B.acc[f * nc + co] + wgt * dl;
-          res[f] = base_value<MIX>(B, f * nc + co) + cst * dl;
+        if (B.stage == 3) {
+          res[f] = fma(wgt, out[f], ac[f]);
         } else {
-          res[f] = B.acc[f * nc + co] + wgt * dl;
+          B.acc[f * nc + co] = fma(wgt, out[f], B.stage == 0 ? ub[f] : ac[f]);
+          res[f] = fma(cst, out[f], ub[f]);
         }
       }
     }
-    bool bad = false;
+    int hmax = 0;  // largest exponent word: infinities and NaN have 0x7ff
 #pragma unroll
-    for (int f = 0; f < 8; f++) bad |= !isfinite(res[f]);
-    if (bad) atomicOr(B.flags, 1);
+    for (int f = 0; f < 8; f++) hmax = max(hmax, __double2hiint(res[f]) & 0x7fffffff);
+    if (hmax >= 0x7ff00000) atomicOr(B.flags, 1);
     int ix[3], iy[3], iz[3];
     ix[0] = gt[0];
     iy[0] = gt[1];
@@ -631,34 +755,40 @@ __global__ void __launch_bounds__(s3::NT, SMAUG_MINB3D) stage3d_fast(const KPara
           const double* r = res;
 #pragma unroll
           for (int f = 0; f < 8; f++) store_value<MIX>(B, f * nc + cc, r[f], is_base);
-          double gg[5];
-          if (a2 == 0 && b == 0 && cz == 0) {
-#pragma unroll
-            for (int f = 0; f < 5; f++) gg[f] = gc[f];
-          } else {
+          // without background fields an image has its source's fast speeds
+          // unless its sign changed
+          if (!BG && (a2 > 0 || b > 0 || cz > 0) && !neg) continue;
+          double gg[5] = {0, 0, 0, 0, 0};
+          if (BG) {
 #pragma unroll
             for (int f = 0; f < 5; f++) gg[f] = __ldg(B.bg + f * nc + cc);
           }
-          double cv[3];
-          cfast3_all(P.gamma, r, gg, cv);
-#pragma unroll
-          for (int d = 0; d < 3; d++) cm[d] = dmax0(cm[d], cv[d]);
+          if (may_exceed<3, BG>(P.gamma, r, gg, cm)) {
+            const double3 cv = cfast3_call(P.gamma, r[0], r[1], r[2], r[3], r[4], r[5], r[6], r[7], gg[0], gg[1],
+                                           gg[2], gg[3], gg[4]);
+            cm[0] = dmax0(cm[0], cv.x);
+            cm[1] = dmax0(cm[1], cv.y);
+            cm[2] = dmax0(cm[2], cv.z);
+          }
         }
   }
+  // maxima above what the grid had when the block started
   __shared__ double red[s3::NT / 32][3];
+  if (__syncthreads_or(cm[0] > seen[0] || cm[1] > seen[1] || cm[2] > seen[2])) {
 #pragma unroll
-  for (int d = 0; d < 3; d++)
-    for (int o = 16; o > 0; o >>= 1) cm[d] = dmax0(cm[d], __shfl_xor_sync(0xffffffffu, cm[d], o));
-  if ((tid & 31) == 0) {
-    red[tid >> 5][0] = cm[0];
-    red[tid >> 5][1] = cm[1];
-    red[tid >> 5][2] = cm[2];
-  }
-  __syncthreads();
-  if (tid < 3) {
-    double v = 0.0;
-    for (int w = 0; w < s3::NT / 32; w++) v = dmax0(v, red[w][tid]);
-    atomicMax(&B.cmax_out[tid], (unsigned long long)__double_as_longlong(v));
+    for (int d = 0; d < 3; d++)
+      for (int o = 16; o > 0; o >>= 1) cm[d] = dmax0(cm[d], __shfl_xor_sync(0xffffffffu, cm[d], o));
+    if ((tid & 31) == 0) {
+      red[tid >> 5][0] = cm[0];
+      red[tid >> 5][1] = cm[1];
+      red[tid >> 5][2] = cm[2];
+    }
+    __syncthreads();
+    if (tid < 3) {
+      double v = 0.0;
+      for (int w = 0; w < s3::NT / 32; w++) v = dmax0(v, red[w][tid]);
+      atomicMax(&B.cmax_out[tid], (unsigned long long)__double_as_longlong(v));
+    }
   }
 }
 
