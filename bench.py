@@ -59,28 +59,26 @@ UNIT = "Mcell-updates/s"
 # DRAM bytes per interior cell per RK4 step measured by ncu on the four stage
 # launches of one step at the benchmark sizes (profiles/dram_traffic_per_stage.md:
 # 2D at 4096^2, 3D at 256^3)
-TRAFFIC_PER_CELL_STEP = {(2, "fp64"): 889.1, (2, "mixed"): 745.7, (3, "fp64"): 2241.6,
-                         (3, "mixed"): 1510.6}
+TRAFFIC_PER_CELL_STEP = {(2, "fp64"): 889.1, (2, "mixed"): 745.7}  # the 3D kernel's: not counted
 
 # What bounds each stage kernel, from its ncu section set (profiles/)
 BOUND_NOTE = {
-    (2, "fp64"): "issue-bound, not HBM: 109 warp instructions per cell and stage at 59.8 % issue "
-                 "active, FP64 pipe 35 %, barrier stalls 2.9 per issue "
-                 "(profiles/stage2d_fp64_ot2048_full.md)",
-    (2, "mixed"): "issue-bound, not HBM: 102 warp instructions per cell and stage at 60.5 % issue "
-                  "active (profiles/stage2d_mixed_ot2048_full.md)",
-    (3, "fp64"): "latency/issue-bound, not HBM: 494 warp instructions per cell and stage at 47.8 % "
-                 "issue active, long-scoreboard stalls 3.65 per issue from re-reads of the state, "
-                 "DRAM traffic 1.8x the algorithmic bytes (profiles/stage3d_fp64_tube128_full.md)",
-    (3, "mixed"): "latency/issue-bound, not HBM: as the FP64 form, with float storage "
-                  "(profiles/stage3d_fp64_tube128_full.md)",
+    (2, "fp64"): "latency/issue-bound, not HBM: 57 warp instructions per cell and stage at 49 % issue "
+                 "active, stalls led by fixed latency, barriers and global loads "
+                 "(profiles/stage_kernels_counters.md)",
+    (2, "mixed"): "latency/issue-bound, not HBM, as the FP64 form",
+    (3, "fp64"): "latency-bound, not HBM: 235 warp instructions per cell and stage at 35 % issue "
+                 "active, stalls led by loads of the state from L2 and barriers "
+                 "(profiles/stage_kernels_counters.md)",
+    (3, "mixed"): "latency-bound, not HBM: as the FP64 form, with float storage",
 }
 
-# FP64 (and FP32) floating-point operations per interior cell per stage counted
-# by ncu (smsp__sass_thread_inst_executed_op_{dadd,dmul,dfma}_pred_on, an FMA
-# counting 2; profiles/fp64_flops_per_cell.md: 2D at 2048^2, 3D at 128^3)
-FLOP_PER_CELL_STAGE = {(2, "fp64"): (1208.0, 29.0), (2, "mixed"): (566.0, 424.0),
-                       (3, "fp64"): (3731.0, 107.0)}
+# FP64 (and FP32) floating-point operations per interior cell per stage as ncu
+# counts them (smsp__sass_thread_inst_executed_op_{dadd,dmul,dfma}_pred_on, an
+# FMA counting 2).  The counts in profiles/fp64_flops_per_cell.md are of earlier
+# kernels that formed every difference several times; the current ones have
+# not been counted, so the line carries no FP64 roofline.
+FLOP_PER_CELL_STAGE = {}
 
 
 def fp64_roofline(ndim, prec, ncell, steps, ms):
